@@ -204,7 +204,8 @@ struct gtb_seq_model {
     std::vector<char> host_stopped_unknown;
     int last_nseg = 0;                           // rows of `logits` that hold segment-last rows (greedy / decode)
     bool use_tensor = true;
-    int tensor_min_rows = 64;
+    int tensor_min_rows = 64;                    // rows from which routed experts run as grouped products and the scan's step sizes from bf16 operands
+    int few_rows = 9;                            // rows from which every other product runs on the tensor cores
     bool use_graph = true;
     bool fused_attn = true;
     bool fused_norm = true;
@@ -294,16 +295,8 @@ template <typename OT>
 int product(gtb_seq_model* m, const void* A, int lda, const bf16* W, int ldw, float* C, int ldc, int M, int N, int Kp, const float* bias, int acc) {
     cudaStream_t st = ctx().stream;
     const OT* a = reinterpret_cast<const OT*>(A);
-    if (sizeof(OT) == 2 && m->use_tensor && M >= m->tensor_min_rows && m->gp) {
-        // An accumulating epilogue reads C one row per thread (the TMEM lane layout): measured 4x the whole product's time.  So the
-        // tensor-core kernel always writes a fresh [M][N] block and a coalesced kernel adds it to the stream.
-        float* dst = (acc && N <= m->cfg.width) ? m->Y : C;
-        int rc = seq_gemm_bf16(m->gp, A, lda, W, ldw, dst, dst == C ? ldc : N, M, N, Kp, bias, dst == C ? acc : 0);
-        if (rc == 0 && dst != C) {
-            const size_t n4 = (size_t)M * N;
-            k_add_block<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(C, ldc, m->Y, N, M);
-            GTB_LAUNCHED();
-        }
+    if (sizeof(OT) == 2 && m->use_tensor && M >= m->few_rows && m->gp) {
+        const int rc = seq_gemm_bf16(m->gp, A, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
         if (rc != -1) return rc;                 // -1: shape not supported by that kernel
     }
     if (M <= 8) {
@@ -1014,7 +1007,7 @@ int run_gated_experts(gtb_seq_model* m, int R, const LayerW& l, bool is_routed, 
     }
     if (l.sff > 0) {
         bool act_done = false;
-        if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->tensor_min_rows && l.sh_inter) {
+        if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->few_rows && l.sh_inter) {
             rc = seq_gemm_bf16_gated(m->gp, opA, wp, l.w_sh_gu, wp, opC, l.sff_p, 0, R, 2 * l.sff, wp, 1, m->shw);
             if (rc > 0) return rc;
             if (rc == 0) { ctx().launches++; act_done = true; }
@@ -1110,7 +1103,7 @@ int run_sandwich_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
     }
     if (l.d.ff_kind == GTB_FF_GELU) {
         bool act_done = false;
-        if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->tensor_min_rows) {
+        if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->few_rows) {
             rc = seq_gemm_bf16_gelu(m->gp, opA, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp);
             if (rc > 0) return rc;
             if (rc == 0) { ctx().launches++; act_done = true; }
@@ -1139,7 +1132,7 @@ int run_sandwich_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
     }
     if (l.d.ff_kind == GTB_FF_SWIGLU) {
         bool act_done = false;
-        if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->tensor_min_rows && l.gu_inter) {
+        if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->few_rows && l.gu_inter) {
             rc = seq_gemm_bf16_gated(m->gp, opA, wp, l.w_gu, wp, opC, l.kfp, 0, R, 2 * l.ff, wp, 1, nullptr);
             if (rc > 0) return rc;
             if (rc == 0) { ctx().launches++; act_done = true; }
@@ -1243,7 +1236,7 @@ int run_prenorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, const
     if (rc) return rc;
     if (l.d.ff_kind == GTB_FF_GEGLU) {
         bool act_done = false;
-        if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->tensor_min_rows && l.gu_inter) {
+        if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->few_rows && l.gu_inter) {
             rc = seq_gemm_bf16_geglu(m->gp, opA, wp, l.w_gu, wp, opC, l.kfp, 0, R, 2 * l.ff, wp);
             if (rc > 0) return rc;
             if (rc == 0) { ctx().launches++; act_done = true; }
@@ -1368,7 +1361,7 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
         bool ff_done = false;
         if (l.ff > 0) {
             // tensor-core pass: gelu(gate) * up comes out of the product's epilogue as the out-projection operand
-            if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->tensor_min_rows && l.gu_inter) {
+            if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->few_rows && l.gu_inter) {
                 rc = seq_gemm_bf16_geglu(m->gp, opB, wp, l.w_gu, wp, opC, l.kout_p, l.kout - l.ff, R, 2 * l.ff, wp);
                 if (rc > 0) return rc;
                 if (rc == 0) { ctx().launches++; ff_done = true; }
@@ -2520,7 +2513,7 @@ int gtb_seq_set_option(gtb_seq_t m, const char* name, int value) {
             if (rc) return rc;
         }
     } else if (n == "tensor") m->use_tensor = value != 0;
-    else if (n == "tensor_min_rows") m->tensor_min_rows = std::max(1, value);
+    else if (n == "tensor_min_rows") m->tensor_min_rows = m->few_rows = std::max(1, value);
     else if (n == "graph") m->use_graph = value != 0;
     else if (n == "fused_attn") m->fused_attn = value != 0;
     else if (n == "fused_norm") m->fused_norm = value != 0;

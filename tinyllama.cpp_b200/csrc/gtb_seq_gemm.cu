@@ -93,7 +93,10 @@ __device__ __forceinline__ float sq_gelu_erf(float z) {
 }
 __device__ __forceinline__ float sq_gate(float z, int kind) { return kind ? sq_silu(z) : sq_gelu(z); }
 
-template <int BN, int EPI>
+// SWAP: 128 rows of W are the M side of the MMA and BN rows of A its N side (tmA is then the map of W, tmB that of A): TMEM lanes are
+// output columns, so the fp32 epilogue writes 128 contiguous bytes per warp and row of C (one row per lane otherwise: 32 half-used sectors per
+// store).  2048 x 6400 x 2048: 54 us against 65; accumulating into C 58 against 762, so residual updates need no block of their own.
+template <int BN, int EPI, bool SWAP>
 __global__ void __launch_bounds__(SQ_THREADS, 1)
 k_seq_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N, int K, const SqEpi ep) {
     using Cfg = SqCfg<BN>;
@@ -110,7 +113,8 @@ k_seq_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     auto bar_tempty = [&](int a) { return bar_base + 8u * (2 * ST + 2 + a); };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_mt = (M + SQ_BM - 1) / SQ_BM, n_nt = (N + BN - 1) / BN;
+    constexpr int TM = SWAP ? BN : SQ_BM, TN = SWAP ? SQ_BM : BN;      // rows and columns of C per tile
+    const int n_mt = (M + TM - 1) / TM, n_nt = (N + TN - 1) / TN;
     const int n_tiles = n_mt * n_nt, nkb = K / SQ_BK;
 
     if (threadIdx.x == 0) {
@@ -135,13 +139,13 @@ k_seq_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                 const int mt = tile % n_mt, nt = tile / n_mt;         // consecutive CTAs share one slice of W
                 const int grp = ep.tile_group ? ep.tile_group[mt] : 0;
                 if (grp < 0) continue;
-                const int wrow = grp * ep.group_rows + nt * BN;
+                const int arow = mt * TM, wrow = grp * ep.group_rows + nt * TN;
                 for (int kb = 0; kb < nkb; kb++) {
                     if (!(ok = sq_wait(bar_empty(s), ph ^ 1, abort_flag))) break;
                     mbar_expect_tx(bar_full(s), Cfg::STAGE_BYTES);
                     const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES;
-                    tma_load_2d(sa, &tmA, bar_full(s), kb * SQ_BK, mt * SQ_BM);
-                    tma_load_2d(sa + Cfg::A_BYTES, &tmB, bar_full(s), kb * SQ_BK, wrow);
+                    tma_load_2d(sa, &tmA, bar_full(s), kb * SQ_BK, SWAP ? wrow : arow);
+                    tma_load_2d(sa + Cfg::A_BYTES, &tmB, bar_full(s), kb * SQ_BK, SWAP ? arow : wrow);
                     if (++s == ST) { s = 0; ph ^= 1; }
                 }
             }
@@ -184,7 +188,28 @@ k_seq_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             tc_fence_after();
             const int row = mt * SQ_BM + lg * 32 + lane;
             const uint32_t tacc = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(as * BN);
-            if (EPI == SQ_EPI_F32) {
+            if (EPI == SQ_EPI_F32 && SWAP) {
+                const int col = nt * TN + lg * 32 + lane, r0 = mt * TM;
+                const float bias = (ep.bias && col < N) ? ep.bias[col] : 0.0f;
+#pragma unroll 1
+                for (int c = chalf * (BN / 64); c < (chalf + 1) * (BN / 64); c++) {
+                    if (r0 + c * 32 >= M) break;
+                    float v[32];
+                    tmem_ld32(tacc + (uint32_t)(c * 32), v);
+                    float* dst = ep.C + (size_t)(r0 + c * 32) * ep.ldc + col;
+                    const int nr = col < N ? min(32, M - r0 - c * 32) : 0;
+                    if (ep.accumulate) {
+                        float p[32];
+#pragma unroll
+                        for (int j = 0; j < 32; j++) p[j] = j < nr ? dst[(size_t)j * ep.ldc] : 0.0f;
+#pragma unroll
+                        for (int j = 0; j < 32; j++) v[j] += p[j];
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (j < nr) dst[(size_t)j * ep.ldc] = v[j] + bias;
+                }
+            } else if (EPI == SQ_EPI_F32) {                         // grouped products: no bias, nothing to add to
 #pragma unroll 1
                 for (int c = chalf * (BN / 64); c < (chalf + 1) * (BN / 64); c++) {
                     const int col = nt * BN + c * 32;
@@ -195,21 +220,11 @@ k_seq_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                         const int nc = min(32, N - col);
                         if (nc == 32 && ((((uintptr_t)dst) & 15) == 0)) {
 #pragma unroll
-                            for (int j = 0; j < 32; j += 4) {
-                                float4 o = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                                if (ep.bias) { o.x += ep.bias[col + j]; o.y += ep.bias[col + j + 1]; o.z += ep.bias[col + j + 2]; o.w += ep.bias[col + j + 3]; }
-                                if (ep.accumulate) { const float4 p = *reinterpret_cast<const float4*>(dst + j); o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w; }
-                                *reinterpret_cast<float4*>(dst + j) = o;
-                            }
+                            for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                         } else {
 #pragma unroll
                             for (int j = 0; j < 32; j++)
-                                if (j < nc) {
-                                    float o = v[j];
-                                    if (ep.bias) o += ep.bias[col + j];
-                                    if (ep.accumulate) o += dst[j];
-                                    dst[j] = o;
-                                }
+                                if (j < nc) dst[j] = v[j];
                         }
                     }
                 }
@@ -289,6 +304,175 @@ k_seq_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
 }
 
+// ------------------------------------------------------------------------------------------------ few rows: swapped operands, split K
+// The same product for passes whose output has too few 128 x BN tiles to occupy the chip (decode batches, short prompts, the head on the
+// wanted rows).  Roles are swapped: 128 rows of W are the M side of the MMA and MT rows of A its N side, so a tile costs no padding beyond a
+// multiple of 16 rows; K is split over the CTAs of a cluster, whose partial sums meet in distributed shared memory in rank order (the
+// result does not depend on timing).  TMEM lanes are output columns, so a warp's partial rows and the final stores are contiguous.
+// Bound by the stream of W: 24 rows x 2048 x 2048 in 4.5 us (8.4 MB: 1.9 TB/s) where the FFMA tile kernel took 120 us; 24 rows x 32000 x 2048
+// in 28 us (131 MB: 4.7 TB/s).
+template <int MT> struct SkCfg {
+    static constexpr uint32_t W_BYTES = 128 * SQ_BK * 2;
+    static constexpr uint32_t A_BYTES = MT * SQ_BK * 2;
+    static constexpr uint32_t STAGE_BYTES = W_BYTES + A_BYTES;
+    static constexpr int STAGES = MT <= 32 ? 5 : 4;      // two CTAs per SM
+    static constexpr uint32_t SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+    static constexpr uint32_t COLS = MT < 32 ? 32 : MT;
+    static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MT >> 3) << 17) | (8u << 24);
+    static_assert(MT * 128 * 4 <= STAGES * STAGE_BYTES, "partial sums reuse the stages");
+};
+constexpr int SK_THREADS = 192;
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int MT, int EPI>
+__global__ void __launch_bounds__(SK_THREADS)
+k_seq_skinny(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA, int M, int N, int K, int cs, const SqEpi ep) {
+    using Cfg = SkCfg<MT>;
+    constexpr int ST = Cfg::STAGES;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + ST * Cfg::STAGE_BYTES);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * ST + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const uint32_t smem_base = smem_u32(smem), bar_base = smem_u32(bars);
+    auto bar_full = [&](int s) { return bar_base + 8u * s; };
+    auto bar_empty = [&](int s) { return bar_base + 8u * (ST + s); };
+    const uint32_t bar_done = bar_base + 8u * (2 * ST);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)blockIdx.x % cs, n0 = (int)blockIdx.x / cs * 128, m0 = (int)blockIdx.y * MT;
+    const int nkb = K / SQ_BK, kb0 = (int)((long long)nkb * rank / cs), kb1 = (int)((long long)nkb * (rank + 1) / cs);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ST; s++) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
+        mbar_init(bar_done, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), Cfg::COLS);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {        // ---------------- TMA producer
+            uint32_t s = 0, ph = 0;
+            for (int kb = kb0; kb < kb1; kb++) {
+                if (!sq_wait(bar_empty(s), ph ^ 1, abort_flag)) break;
+                mbar_expect_tx(bar_full(s), Cfg::STAGE_BYTES);
+                const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES;
+                tma_load_2d(sw, &tmW, bar_full(s), kb * SQ_BK, n0);
+                tma_load_2d(sw + Cfg::W_BYTES, &tmA, bar_full(s), kb * SQ_BK, m0);
+                if (++s == ST) { s = 0; ph ^= 1; }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {        // ---------------- MMA issuer
+            uint32_t s = 0, ph = 0;
+            bool ok = true;
+            for (int kb = kb0; kb < kb1; kb++) {
+                if (!(ok = sq_wait(bar_full(s), ph, abort_flag))) break;
+                tc_fence_after();
+                const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES, sa = sw + Cfg::W_BYTES;
+#pragma unroll
+                for (int k = 0; k < SQ_BK / 16; k++)
+                    umma_f16(tmem_base, umma_desc_sw128(sw + k * 32), umma_desc_sw128(sa + k * 32), Cfg::IDESC, kb > kb0 || k > 0);
+                umma_commit(bar_empty(s));
+                if (++s == ST) { s = 0; ph ^= 1; }
+            }
+            if (ok) umma_commit(bar_done);
+        }
+        __syncwarp();
+    } else {                    // ---------------- accumulator -> partial[row of A][128 output columns]
+        const bool ok = sq_wait(bar_done, 0, abort_flag);
+        tc_fence_after();
+        if (ok) {
+            const int lg = warp & 3;
+            float* part = reinterpret_cast<float*>(smem) + lg * 32 + lane;
+#pragma unroll 1
+            for (int c = 0; c < MT; c += 16) {
+                if (m0 + c >= M) break;
+                float v[16];
+                tmem_ld16(tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)c, v);
+#pragma unroll
+                for (int j = 0; j < 16; j++) part[(c + j) * 128] = v[j];
+            }
+        }
+        tc_fence_before();
+    }
+    if (cs > 1) cluster_sync_all();
+    else __syncthreads();
+    // every CTA of the cluster finishes its share of the tile's rows
+    const int rows = min(MT, M - m0), r0 = rows * rank / cs, r1 = rows * (rank + 1) / cs;
+    constexpr int Q = EPI == SQ_EPI_GEGLU ? 16 : 32;       // groups of four outputs per row
+    auto sum4 = [&](int m, int n) {
+        const uint32_t a = smem_base + (uint32_t)(m * 128 + n) * 4;
+        if (cs == 1) return *reinterpret_cast<const float4*>(smem + (size_t)(m * 128 + n) * 4);
+        float4 s = ld_cluster_f4(a, 0);
+        for (int p = 1; p < cs; p++) { const float4 v = ld_cluster_f4(a, p); s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
+        return s;
+    };
+    for (int i = threadIdx.x; i < (r1 - r0) * Q; i += SK_THREADS) {
+        const int m = r0 + i / Q, q = i % Q, row = m0 + m;
+        if (EPI == SQ_EPI_F32) {
+            const int n = n0 + q * 4;
+            if (n >= N) continue;
+            float4 o = sum4(m, q * 4);
+            float* dst = ep.C + (size_t)row * ep.ldc + n;
+            if (n + 4 <= N && (((uintptr_t)dst) & 15) == 0) {
+                if (ep.bias) { o.x += ep.bias[n]; o.y += ep.bias[n + 1]; o.z += ep.bias[n + 2]; o.w += ep.bias[n + 3]; }
+                if (ep.accumulate) { const float4 p = *reinterpret_cast<const float4*>(dst); o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w; }
+                *reinterpret_cast<float4*>(dst) = o;
+            } else {
+                const float v[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (n + j < N) dst[j] = v[j] + (ep.bias ? ep.bias[n + j] : 0.0f) + (ep.accumulate ? dst[j] : 0.0f);
+            }
+        } else {
+            // (columns beyond the product's come out as zeros: the operand's padding, as far as the tile reaches, is written too)
+            const int c = (EPI == SQ_EPI_GEGLU ? n0 >> 1 : n0) + q * 4, nc = ep.ld_act - ep.act_off;
+            if (c >= nc) continue;
+            float v[4];
+            if (EPI == SQ_EPI_GEGLU) {
+                const int g = (q >> 3) * 64 + (q & 7) * 4;                // 32 gate columns, then their 32 up columns
+                const float4 a = sum4(m, g), u = sum4(m, g + 32);
+                const float wt = ep.row_w ? ep.row_w[row] : 1.0f;
+                v[0] = wt * sq_gate(a.x, ep.act_kind) * u.x; v[1] = wt * sq_gate(a.y, ep.act_kind) * u.y;
+                v[2] = wt * sq_gate(a.z, ep.act_kind) * u.z; v[3] = wt * sq_gate(a.w, ep.act_kind) * u.w;
+            } else {
+                const float4 a = sum4(m, q * 4);
+                v[0] = sq_gelu_erf(a.x); v[1] = sq_gelu_erf(a.y); v[2] = sq_gelu_erf(a.z); v[3] = sq_gelu_erf(a.w);
+            }
+            __nv_bfloat16* dst = ep.act + (size_t)row * ep.ld_act + ep.act_off + c;
+            if (c + 4 <= nc && (((uintptr_t)dst) & 7) == 0) {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+                *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (c + j < nc) dst[j] = __float2bfloat16_rn(v[j]);
+            }
+        }
+    }
+    if (cs > 1) cluster_sync_all();       // a peer may still be reading this CTA's partial sums
+    if (threadIdx.x == 0 && *abort_flag && ep.status) atomicExch(ep.status, 1);
+    if (warp == 1) tmem_dealloc(tmem_base, Cfg::COLS);
+}
+
 // ---------------------------------------------------------------------------------------------------------------- host
 typedef CUresult (*PFN_tmapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                         const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -297,7 +481,8 @@ typedef CUresult (*PFN_tmapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuin
 struct SeqGemmPlan {
     PFN_tmapEncodeTiled enc = nullptr;
     int* d_status = nullptr;
-    bool attr[2][4] = {{false, false, false, false}, {false, false, false, false}};
+    bool attr[2][2][4] = {};
+    bool sk_attr[3][4] = {};
 };
 
 int seq_gemm_create(SeqGemmPlan** out) {
@@ -337,35 +522,103 @@ static int make_map(SeqGemmPlan* p, CUtensorMap* m, const void* base, int rows, 
     return GTB_OK;
 }
 
-template <int BN, int EPI>
+template <int BN, int EPI, bool SWAP = false>
 static int launch(SeqGemmPlan* p, const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, const SqEpi& ep) {
     using Cfg = SqCfg<BN>;
-    bool& attr = p->attr[BN == 256][EPI];
+    bool& attr = p->attr[SWAP][BN == 256][EPI];
     if (!attr) {
-        GTB_CUDA(cudaFuncSetAttribute(k_seq_gemm<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
+        GTB_CUDA(cudaFuncSetAttribute(k_seq_gemm<BN, EPI, SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
         attr = true;
     }
-    const int n_tiles = ((M + SQ_BM - 1) / SQ_BM) * ((N + BN - 1) / BN);
+    constexpr int TM = SWAP ? BN : SQ_BM, TN = SWAP ? SQ_BM : BN;
+    const int n_tiles = ((M + TM - 1) / TM) * ((N + TN - 1) / TN);
     const int grid = n_tiles < ctx().sm_count ? n_tiles : ctx().sm_count;
-    k_seq_gemm<BN, EPI><<<grid, SQ_THREADS, Cfg::SMEM, ctx().stream>>>(ta, tb, M, N, K, ep);
+    k_seq_gemm<BN, EPI, SWAP><<<grid, SQ_THREADS, Cfg::SMEM, ctx().stream>>>(ta, tb, M, N, K, ep);
     GTB_LAUNCHED();
     return GTB_OK;
 }
 
+template <int MT, int EPI>
+static int launch_skinny(bool& attr, const CUtensorMap& tw, const CUtensorMap& ta, int M, int N, int K, int cs, const SqEpi& ep) {
+    using Cfg = SkCfg<MT>;
+    if (!attr) {
+        GTB_CUDA(cudaFuncSetAttribute(k_seq_skinny<MT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
+        attr = true;
+    }
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3((N + 127) / 128 * cs, (M + MT - 1) / MT);
+    lc.blockDim = dim3(SK_THREADS);
+    lc.dynamicSmemBytes = Cfg::SMEM;
+    lc.stream = ctx().stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    GTB_CUDA(cudaLaunchKernelEx(&lc, k_seq_skinny<MT, EPI>, tw, ta, M, N, K, cs, ep));
+    GTB_LAUNCHED();
+    return GTB_OK;
+}
+template <int EPI>
+static int launch_skinny_mt(SeqGemmPlan* p, int mt, const CUtensorMap& tw, const CUtensorMap& ta, int M, int N, int K, int cs, const SqEpi& ep) {
+    if (mt == 16) return launch_skinny<16, EPI>(p->sk_attr[0][EPI], tw, ta, M, N, K, cs, ep);
+    if (mt == 32) return launch_skinny<32, EPI>(p->sk_attr[1][EPI], tw, ta, M, N, K, cs, ep);
+    return launch_skinny<64, EPI>(p->sk_attr[2][EPI], tw, ta, M, N, K, cs, ep);
+}
+
+// Which kernel takes an M x N product.  Few rows mean few tiles, and a CTA streams W at a fixed rate however short its tile is: cutting K is
+// what brings the chip's bandwidth to bear, until about two CTAs per SM are resident (beyond that the further clusters wait for a second
+// wave) or a CTA's share of K is too short to pay for its start.  So the split-K kernel takes a product as long as K can be cut in two within
+// that many CTAs, and every product of up to 64 rows (one tile row: nothing to gain from persistence).  Measured cold, launch included:
+// N = K = 2048, 24 rows: 18.5 / 15.3 / 13.2 us for 1 / 2 / 4 cuts; N = 6400, 40 rows: 20.6 / 18.4 / 16.8; N = 32000, 24 rows: 36.8 / 41.1 / 48.5;
+// against the persistent kernel with 128 rows (N = K = 2048): 14.9 to 19.2, with 512 rows 19.1 to 20.5, with 800 rows 28.9 to 20.6.
+struct SkChoice { int mt = 0, cs = 1; };
+static SkChoice skinny_choice(int M, int N, int K) {
+    SkChoice c;
+    const int nt = (N + 127) / 128, slots = 2 * ctx().sm_count - 40, nkb = K / SQ_BK;
+    int mt = M <= 16 ? 16 : M <= 32 ? 32 : 64;
+    if (mt == 64 && M <= 64 && nt * 2 <= 64) mt = 32;
+    const int tiles = nt * ((M + mt - 1) / mt);
+    if (tiles * 2 > slots && M > 64) return c;
+    c.mt = mt;
+    while (c.cs < 8 && tiles * c.cs * 2 <= slots && nkb >= c.cs * 4) c.cs *= 2;
+    return c;
+}
+
 static int run(SeqGemmPlan* p, int epi, const void* A, int lda, const void* W, int ldw, int M, int N, int K, const SqEpi& ep) {
     if (!p || K <= 0 || (K % SQ_BK) || (lda % 8) || (ldw % 8) || (((uintptr_t)A | (uintptr_t)W) & 15)) return -1;
+    CUtensorMap ta, tb;
+    int rc;
+    const SkChoice sk = skinny_choice(M, N, K);
+    if (sk.mt) {
+        rc = make_map(p, &tb, W, N, K, ldw, 128);
+        if (rc) return rc;
+        rc = make_map(p, &ta, A, M, K, lda, sk.mt);
+        if (rc) return rc;
+        if (epi == SQ_EPI_GELU) return launch_skinny_mt<SQ_EPI_GELU>(p, sk.mt, tb, ta, M, N, K, sk.cs, ep);
+        if (epi == SQ_EPI_F32) return launch_skinny_mt<SQ_EPI_F32>(p, sk.mt, tb, ta, M, N, K, sk.cs, ep);
+        return launch_skinny_mt<SQ_EPI_GEGLU>(p, sk.mt, tb, ta, M, N, K, sk.cs, ep);
+    }
+    if (epi == SQ_EPI_F32) {
+        // 128-row tiles of A while one wave holds them all (half the MMA rate, but twice the SMs) or no second tile is needed, 256-row tiles
+        // beyond (N = 5632, K = 1024, cold: 384 rows 16.3 against 17.7 us, 512 rows 21.2 against 17.8)
+        const int bn = M <= 128 || ((M + 127) / 128) * ((N + 127) / 128) <= ctx().sm_count ? 128 : 256;
+        rc = make_map(p, &tb, W, N, K, ldw, SQ_BM);
+        if (rc) return rc;
+        rc = make_map(p, &ta, A, M, K, lda, bn);
+        if (rc) return rc;
+        return bn == 256 ? launch<256, SQ_EPI_F32, true>(p, tb, ta, M, N, K, ep) : launch<128, SQ_EPI_F32, true>(p, tb, ta, M, N, K, ep);
+    }
     // 256-wide tiles when they still give every SM a tile; otherwise 128-wide
     const int mt = (M + SQ_BM - 1) / SQ_BM;
     // (the 128-wide MMA reads as much of A from shared memory per FLOP as the 256-wide one reads of A and W together: it runs at about
     // half the rate, so it only pays when 256-wide tiles would leave most SMs idle)
     const int bn = (N > 128 && mt * ((N + 255) / 256) * 2 >= ctx().sm_count) ? 256 : 128;
-    CUtensorMap ta, tb;
-    int rc = make_map(p, &ta, A, M, K, lda, SQ_BM);
+    rc = make_map(p, &ta, A, M, K, lda, SQ_BM);
     if (rc) return rc;
     rc = make_map(p, &tb, W, N, K, ldw, bn);
     if (rc) return rc;
     if (epi == SQ_EPI_GELU) return bn == 256 ? launch<256, SQ_EPI_GELU>(p, ta, tb, M, N, K, ep) : launch<128, SQ_EPI_GELU>(p, ta, tb, M, N, K, ep);
-    if (epi == SQ_EPI_F32) return bn == 256 ? launch<256, SQ_EPI_F32>(p, ta, tb, M, N, K, ep) : launch<128, SQ_EPI_F32>(p, ta, tb, M, N, K, ep);
     return bn == 256 ? launch<256, SQ_EPI_GEGLU>(p, ta, tb, M, N, K, ep) : launch<128, SQ_EPI_GEGLU>(p, ta, tb, M, N, K, ep);
 }
 

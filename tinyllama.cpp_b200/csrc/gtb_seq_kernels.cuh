@@ -647,13 +647,6 @@ __global__ void k_geglu(const float* __restrict__ G, int ff, OT* __restrict__ ou
     const int gc = interleaved ? (c >> 5) * 64 + (c & 31) : c, uc = interleaved ? gc + 32 : ff + c;
     out[(size_t)r * ld_out + a_off + c] = cvt<OT>(gelu_tanh(G[(size_t)r * 2 * ff + gc]) * G[(size_t)r * 2 * ff + uc]);
 }
-// C[r][c] += Y[r][c] for an [M][N] block (N contiguous in Y)
-__global__ void k_add_block(float* __restrict__ C, int ldc, const float* __restrict__ Y, int N, int M) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)M * N) return;
-    const size_t r = i / N, c = i % N;
-    C[r * ldc + c] += Y[i];
-}
 // operand [x | x0] of the loop's entry projection
 template <typename OT>
 __global__ void k_concat2(const float* __restrict__ x, const float* __restrict__ x0, int width, OT* __restrict__ out, int ld_out) {
