@@ -23,12 +23,12 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-O2", "--expt-relaxed-constexpr",
 ]
 SEQ_LIB = HERE / "libgten_b200_seq.so"
-SEQ_SOURCES = ["gtb_api.cu", "gtb_seq.cu", "gtb_seq_gemm.cu"]
+SEQ_SOURCES = ["gtb_api.cu", "gtb_seq.cu", "gtb_seq_gemm.cu", "gtb_seq_attn.cu"]
 # the sequence models have no bit-exact contract with a CPU program: fused multiply-adds are welcome (gtb_api.cu keeps the flag)
 SEQ_FLAGS = [f for f in NVCC_FLAGS if f != "-fmad=false"]
 TARGETS = {
     "llama": (LIB, SOURCES, {}),
-    "seq": (SEQ_LIB, SEQ_SOURCES, {"gtb_seq.cu": SEQ_FLAGS, "gtb_seq_gemm.cu": SEQ_FLAGS}),
+    "seq": (SEQ_LIB, SEQ_SOURCES, {s: SEQ_FLAGS for s in SEQ_SOURCES[1:]}),
 }
 
 

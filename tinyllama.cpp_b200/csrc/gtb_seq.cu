@@ -34,6 +34,7 @@
 #include "../../include/gten_b200_seq.h"
 #include "gtb_internal.h"
 #include "gtb_sample.cuh"
+#include "gtb_seq_attn.h"
 #include "gtb_seq_gemm.h"
 #include "gtb_seq_kernels.cuh"
 #include "gtb_seq_mixers.cuh"
@@ -349,7 +350,22 @@ int launch_sigattn_mma(const PassTables& t, const AttnBranch& a, int S, int n_ti
     GTB_LAUNCHED();
     return GTB_OK;
 }
-int sigattn_mma(const PassTables& t, const AttnBranch& a, int S, int n_tiles, const float* P, int ldp, const bf16* kc, const bf16* vc, bf16* out, int ld_out) {
+// what both attention kinds hand to the tcgen05 kernel (tiles of 128 rows: at most (tiles of 64 rows + segments) / 2 of them)
+AttnTc attn_tc_args(const gtb_seq_model* m, const PassTables& t, int S, const float* Q, int ldq, int q_off, const bf16* kc, const bf16* vc, bf16* out, int ld_out, int a_off) {
+    AttnTc x{};
+    x.seg_slot = t.seg_slot; x.seg_row0 = t.seg_row0; x.seg_len = t.seg_len; x.row_pos = t.row_pos; x.S = S;
+    x.Q = Q; x.ldq = ldq; x.q_off = q_off; x.kc = kc; x.vc = vc; x.max_ctx = m->cfg.max_ctx; x.cache_rows = m->cfg.n_slots * m->cfg.max_ctx;
+    x.maps = 1; x.gsrc = Q; x.out = out; x.ld_out = ld_out; x.a_off = a_off;
+    return x;
+}
+int sigattn_mma(const gtb_seq_model* m, const PassTables& t, const AttnBranch& a, int S, int n_tiles, const float* P, int ldp, const bf16* kc, const bf16* vc, bf16* out, int ld_out) {
+    if (m->use_tensor) {
+        AttnTc x = attn_tc_args(m, t, S, P, ldp, a.q_off, kc, vc, out, ld_out, a.a_off);
+        x.heads = a.heads; x.kv_heads = a.kv_heads; x.dim = a.dim; x.vdim = a.vdim; x.ld_k = a.kv_heads * a.dim; x.ld_v = a.kv_heads * a.vdim;
+        x.scale = a.scale; x.sigmoid = 1; x.pb = a.pb; x.out_scale = a.out_scale;
+        const int rc = seq_attn_tc(m->gp, x, (n_tiles + S) / 2);
+        if (rc != -1) return rc;
+    }
     const int dp = a.dim <= 32 ? 32 : a.dim <= 64 ? 64 : 128, vp = a.vdim <= 32 ? 32 : a.vdim <= 64 ? 64 : 128;
     // (HPC = 2 -- two query heads of a group sharing a CTA's K/V tiles -- was measured equal to one head per CTA at 32 heads x 2048 rows)
 #define SA_CASE(D, V) if (dp == D && vp == V) return launch_sigattn_mma<D, V, 1>(t, a, S, n_tiles, P, ldp, kc, vc, out, ld_out)
@@ -382,8 +398,19 @@ int launch_sattn_mma(const PassTables& t, const SoftAttn& a, int S, int n_tiles,
     return GTB_OK;
 }
 // out_f != null: the units' outputs go there in fp32 ([rows][ld_f], unit-major) without gate or weight instead of `out`
-int sattn_mma(const PassTables& t, const SoftAttn& a, int S, int n_tiles, const float* P, int ldp, const bf16* kc, const bf16* vc, const float* pk, const float* pv,
-              bf16* out, int ld_out, float* out_f = nullptr, int ld_f = 0) {
+int sattn_mma(const gtb_seq_model* m, const PassTables& t, const SoftAttn& a, int S, int n_tiles, const float* P, int ldp, const bf16* kc, const bf16* vc, const float* pk,
+              const float* pv, bf16* out, int ld_out, float* out_f = nullptr, int ld_f = 0) {
+    if (m->use_tensor && a.pool <= 0 && a.keep <= 0) {
+        AttnTc x = attn_tc_args(m, t, S, P, ldp, a.q_off, kc, vc, out, ld_out, a.a_off);
+        x.heads = a.heads; x.maps = sa_maps(a); x.kv_heads = a.kv_heads; x.dim = a.dim; x.vdim = a.vdim;
+        x.ld_k = a.kv_heads * x.maps * a.dim; x.ld_v = a.kv_heads * a.vdim;
+        x.scale = a.scale; x.softcap = a.softcap; x.window = a.window; x.chunk = a.chunk; x.sink = a.sink; x.slope = a.slope;
+        x.out_scale = a.out_scale != 0.0f ? a.out_scale : 1.0f;
+        x.gate = a.gate; x.gsrc = a.gate_src ? a.gate_src : P; x.g_ld = a.gate_src ? a.gate_ld : ldp; x.g_off = a.g_off;
+        x.out_f = out_f; x.ld_f = ld_f;
+        const int rc = seq_attn_tc(m->gp, x, (n_tiles + S) / 2);
+        if (rc != -1) return rc;
+    }
     const int dp = a.dim <= 32 ? 32 : a.dim <= 64 ? 64 : 128, vp = a.vdim <= 32 ? 32 : a.vdim <= 64 ? 64 : 128;
 #define SA_CASE(D, V) if (dp == D && vp == V) return launch_sattn_mma<D, V>(t, a, S, n_tiles, P, ldp, kc, vc, pk, pv, out, ld_out, out_f, ld_f)
     SA_CASE(32, 32); SA_CASE(32, 64); SA_CASE(32, 128); SA_CASE(64, 32); SA_CASE(64, 64); SA_CASE(64, 128); SA_CASE(128, 32); SA_CASE(128, 64); SA_CASE(128, 128);
@@ -453,7 +480,7 @@ int run_postnorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
         }
         int done = -1;
         if (portions && sizeof(OT) == 2 && a.dim <= 128 && a.vdim <= 128)
-            done = sattn_mma(t, a, S, n_qtiles, m->P, l.n1, (const bf16*)run.kc[0], (const bf16*)run.vc[0], run.pk, run.pv, (bf16*)opC, l.kout_p);
+            done = sattn_mma(m, t, a, S, n_qtiles, m->P, l.n1, (const bf16*)run.kc[0], (const bf16*)run.vc[0], run.pk, run.pv, (bf16*)opC, l.kout_p);
         if (done > 0) return done;
         if (done < 0 && !portions && R <= SPLIT_MAX_ROWS && m->sattn_part) {
             // decode rows: one CTA per 128 keys of the longest key list this layer can meet (window tokens + pooled blocks), at most 32
@@ -673,7 +700,7 @@ int run_soft_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const R
     const size_t smem = (a.dim + 128 + 33) * sizeof(float);
     int done = -1;
     if (portions && sizeof(OT) == 2 && a.dim <= 128 && a.vdim <= 128)
-        done = sattn_mma(t, a, S, n_qtiles, Q, ldq, (const bf16*)run.kc[bi], (const bf16*)run.vc[bi], nullptr, nullptr, (bf16*)opC, l.kout_p, of, ldf);
+        done = sattn_mma(m, t, a, S, n_qtiles, Q, ldq, (const bf16*)run.kc[bi], (const bf16*)run.vc[bi], nullptr, nullptr, (bf16*)opC, l.kout_p, of, ldf);
     if (done > 0) return done;
     if (done < 0 && !portions && R <= SPLIT_MAX_ROWS && m->sattn_part) {
         int max_keys = c.max_ctx;
@@ -942,7 +969,7 @@ int run_latent_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const
         SoftAttn sa{};
         sa.heads = sa.kv_heads = a.heads; sa.dim = hd; sa.vdim = a.vdim; sa.scale = b.d.scale; sa.eps = c.eps; sa.window = b.d.window; sa.sink = b.d_sink;
         sa.gate = b.d.gated; sa.q_off = 0; sa.gate_src = m->P; sa.gate_ld = l.n1; sa.g_off = b.g_off; sa.a_off = b.a_off; sa.own_kv = 1; sa.max_ctx = c.max_ctx;
-        rc = sattn_mma(t, sa, S, n_qtiles, m->latQ, ld_qr, m->latKx, m->latVx, nullptr, nullptr, (bf16*)opC, l.kout_p);
+        rc = sattn_mma(m, t, sa, S, n_qtiles, m->latQ, ld_qr, m->latKx, m->latVx, nullptr, nullptr, (bf16*)opC, l.kout_p);
         if (rc < 0) return gtb::fail(GTB_ERR_STATE, "head sizes outside the tiled attention kernel");
         return rc;
     }
@@ -1379,7 +1406,7 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
                 GTB_LAUNCHED();
                 int done = -1;
                 if (portions && sizeof(OT) == 2 && a.dim <= 128 && a.vdim <= 128)
-                    done = sigattn_mma(t, a, S, n_qtiles, m->P, l.n1, (const bf16*)run.kc[bi], (const bf16*)run.vc[bi], (bf16*)opC, l.kout_p);
+                    done = sigattn_mma(m, t, a, S, n_qtiles, m->P, l.n1, (const bf16*)run.kc[bi], (const bf16*)run.vc[bi], (bf16*)opC, l.kout_p);
                 if (done > 0) return done;
                 if (done < 0 && !portions && m->attn_splits > 1 && R <= SPLIT_MAX_ROWS) {
                     // (a group-major variant -- one CTA scoring a key for all query heads of its K/V head -- was measured slower at 32 heads

@@ -25,6 +25,7 @@
 #include <cuda_bf16.h>
 
 #include "gtb_internal.h"
+#include "gtb_seq_gemm_plan.h"
 #include "gtb_tc.cuh"
 
 namespace gtb {
@@ -474,17 +475,6 @@ k_seq_skinny(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
 }
 
 // ---------------------------------------------------------------------------------------------------------------- host
-typedef CUresult (*PFN_tmapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                        const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                        CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-struct SeqGemmPlan {
-    PFN_tmapEncodeTiled enc = nullptr;
-    int* d_status = nullptr;
-    bool attr[2][2][4] = {};
-    bool sk_attr[3][4] = {};
-};
-
 int seq_gemm_create(SeqGemmPlan** out) {
     *out = nullptr;
     void* p = nullptr;
