@@ -1,13 +1,16 @@
 // gtb_seq_attn.cu -- attention of prompt portions (bf16 mode) on the 5th-generation tensor cores: softmax attention under a causal, windowed or
 // chunked mask with an optional sink, soft cap and distance slope, and sigmoid attention.
 //
-// A CTA owns 128 consecutive rows of one segment and one query unit; two CTAs share an SM, so that one's products run while the other's weights
-// are computed.  Warps 0-3 hold one row per thread (TMEM lane = row): scores from TMEM, mask, weights in fp32, bf16 weights back to TMEM.
-// Warp 4 loads key and value tiles by TMA (128-byte swizzle), one thread of warp 5 issues the products:
-//     S[128][KT] = Q K^T      (Q staged once as bf16 in shared memory, K tile K-major)
+// A CTA owns 128 consecutive rows of one segment and one query unit; two CTAs share an SM.  Warps 0-3 hold one row per thread (TMEM lane =
+// row): scores from TMEM, mask, weights in fp32, bf16 weights back to TMEM.  Warp 4 loads key and value tiles by TMA (128-byte swizzle), one
+// thread of warp 5 issues the products:
+//     S[128][64] = Q K^T      (Q staged once as bf16 in shared memory, K tile K-major)
 //     O[128][VP] += P V       (P bf16 from TMEM, V tile as it lies in the cache: rows of keys, the MN-major B operand)
-// The softmax keeps its reference maximum until a row's scores exceed it by 2^8 and only then rescales O in TMEM (a rare event; weights up
-// to 2^8 lose nothing in fp32 sums or bf16 operands).  Scores, weights, sums and the output are fp32, the weights enter P V as bf16.
+// There are two score buffers, and the weights of a tile replace its scores: while tile j's weights are computed, P V of tile j - 1 and the
+// scores of tile j + 1 run, so the weight threads hardly ever wait for a product's latency.
+// The softmax keeps its reference maximum until a row's scores exceed it by 2^8 and only then rescales O in TMEM (a rare event, the only one
+// that waits for P V; weights up to 2^8 lose nothing in fp32 sums or bf16 operands).  Scores, weights, sums and the output are fp32, the
+// weights enter P V as bf16.
 //
 // Bound: the weights' exponentials (16 per clock and SM; a 128 x 128 tile takes 1024 cycles, its two products 512).
 //
@@ -25,16 +28,17 @@
 namespace gtb {
 namespace seq {
 
-constexpr int AT_THREADS = 192, AT_STAGES = 2;
+constexpr int AT_THREADS = 192;
 
+constexpr int AT_KT = 64;                         // keys per tile
 template <int DP, int VP> struct AtCfg {
-    static constexpr int KT = (DP == 64 && VP == 64) ? 128 : 64;          // keys per tile
-    static constexpr uint32_t Q_BYTES = 128 * DP * 2, K_BYTES = KT * DP * 2, V_BYTES = KT * VP * 2;
-    static constexpr uint32_t SMEM = Q_BYTES + AT_STAGES * (K_BYTES + V_BYTES) + 1024 + 256;
-    // TMEM columns: scores, weights (two per column), output
-    static constexpr uint32_t COLS = 256, P_COL = KT, O_COL = KT == 128 ? 192 : 128;
-    static_assert(P_COL + KT / 2 <= O_COL && O_COL + VP <= COLS, "TMEM columns");
-    static constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KT >> 3) << 17) | (8u << 24);
+    static constexpr int STAGES = DP + VP == 256 ? 2 : 3;      // (two CTAs per SM)
+    static constexpr uint32_t Q_BYTES = 128 * DP * 2, K_BYTES = AT_KT * DP * 2, V_BYTES = AT_KT * VP * 2;
+    static constexpr uint32_t SMEM = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + 1024 + 256;
+    // TMEM columns: two score buffers (a tile's weights, two per column, replace its scores), output
+    static constexpr uint32_t COLS = 256, O_COL = 2 * AT_KT;
+    static_assert(O_COL + VP <= COLS, "TMEM columns");
+    static constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(AT_KT >> 3) << 17) | (8u << 24);
     static constexpr uint32_t IDESC_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (8u << 17) | (8u << 24);      // B MN-major, N = 64
 };
 
@@ -78,6 +82,11 @@ __device__ __forceinline__ uint32_t at_pack(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&v);
 }
+__device__ __forceinline__ float at_max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
 // every lane of the warp gets the same answer
 __device__ __forceinline__ bool at_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     bool ok = false;
@@ -93,11 +102,12 @@ template <int DP, int VP, bool SIG>
 __global__ void __launch_bounds__(AT_THREADS, 2)
 k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const AttnTc a, int* status) {
     using Cfg = AtCfg<DP, VP>;
-    constexpr int KT = Cfg::KT;
+    constexpr int KT = AT_KT, AT_STAGES = Cfg::STAGES;
     extern __shared__ unsigned char smem_raw[];
-    // the CTA's tile: 128 rows of a segment; a segment's last tiles sweep the most keys and start first
+    // the CTA's tile: 128 rows of a segment.  Tiles are the slow grid dimension and a segment's last tiles, which sweep the most keys, come
+    // first: every unit's longest tiles start before any shorter one
     int seg = -1, q0 = 0;
-    for (int s = 0, idx = blockIdx.x; s < a.S; s++) {
+    for (int s = 0, idx = blockIdx.y; s < a.S; s++) {
         const int n = (a.seg_len[s] + 127) / 128;
         if (idx < n) { seg = s; q0 = (n - 1 - idx) * 128; break; }
         idx -= n;
@@ -106,17 +116,21 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sm_q = smem_u32(smem), sm_k = sm_q + Cfg::Q_BYTES, sm_v = sm_k + AT_STAGES * Cfg::K_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::Q_BYTES + AT_STAGES * (Cfg::K_BYTES + Cfg::V_BYTES));
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 * AT_STAGES + 3);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 * AT_STAGES + 7);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t bb = smem_u32(bars);
     auto k_full = [&](int s) { return bb + 8u * s; };
     auto k_empty = [&](int s) { return bb + 8u * (AT_STAGES + s); };
     auto v_full = [&](int s) { return bb + 8u * (2 * AT_STAGES + s); };
     auto v_empty = [&](int s) { return bb + 8u * (3 * AT_STAGES + s); };
-    const uint32_t s_bar = bb + 8u * (4 * AT_STAGES), p_bar = s_bar + 8, o_bar = s_bar + 16;
+    // per score buffer: scores there, weights there, P V done; one for the staged queries
+    auto s_bar = [&](int j) { return bb + 8u * (4 * AT_STAGES + (j & 1)); };
+    auto p_bar = [&](int j) { return bb + 8u * (4 * AT_STAGES + 2 + (j & 1)); };
+    auto o_bar = [&](int j) { return bb + 8u * (4 * AT_STAGES + 4 + (j & 1)); };
+    const uint32_t q_bar = bb + 8u * (4 * AT_STAGES + 6);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int u = blockIdx.y, hd = u / a.maps, g = hd / (a.heads / a.kv_heads), ku = g * a.maps + u % a.maps;
+    const int u = blockIdx.x, hd = u / a.maps, g = hd / (a.heads / a.kv_heads), ku = g * a.maps + u % a.maps;
     const int slot = a.seg_slot[seg], row0 = a.seg_row0[seg] + q0, nq = min(128, a.seg_len[seg] - q0);
     const int pos0 = a.row_pos[row0], last = pos0 + nq - 1;
     auto first_key = [&](int pos) {
@@ -128,31 +142,12 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < 4 * AT_STAGES; s++) mbar_init(bb + 8u * s, 1);
-        mbar_init(s_bar, 1); mbar_init(p_bar, 128); mbar_init(o_bar, 1);
+        for (int j = 0; j < 2; j++) { mbar_init(s_bar(j), 1); mbar_init(p_bar(j), 128); mbar_init(o_bar(j), 1); }
+        mbar_init(q_bar, 128);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 5) tmem_alloc(smem_u32(tmem_slot), Cfg::COLS);
-    // queries -> bf16, 128-byte swizzle, one 64-column tile after the other; the sign of the scale rides on them
-    const float sgn = a.scale < 0.0f ? -1.0f : 1.0f;
-    for (int e = threadIdx.x; e < 128 * (DP / 8); e += AT_THREADS) {
-        const int r = e / (DP / 8), c8 = e % (DP / 8);
-        uint4 w = make_uint4(0, 0, 0, 0);
-        if (r < nq) {
-            const float* src = a.Q + (size_t)(row0 + r) * a.ldq + a.q_off + u * DP + c8 * 8;
-            float v[8];
-            if ((((uintptr_t)src) & 15) == 0) {
-                const float4 x = *reinterpret_cast<const float4*>(src), y = *reinterpret_cast<const float4*>(src + 4);
-                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = src[j];
-            }
-            w = make_uint4(at_pack(v[0] * sgn, v[1] * sgn), at_pack(v[2] * sgn, v[3] * sgn), at_pack(v[4] * sgn, v[5] * sgn), at_pack(v[6] * sgn, v[7] * sgn));
-        }
-        *reinterpret_cast<uint4*>(smem + (c8 >> 3) * (128 * 128) + r * 128 + (((c8 & 7) ^ (r & 7)) << 4)) = w;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -160,8 +155,6 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
 
     if (warp == 4) {
         if (lane == 0) {            // ---------------- TMA producer
-            tma_prefetch_desc(&tmK);
-            tma_prefetch_desc(&tmV);
             auto wait1 = [&](uint32_t bar, uint32_t parity) {
                 for (int it = 0; it < (1 << 24); it++) {
                     if (mbar_try_wait(bar, parity)) return true;
@@ -183,52 +176,84 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
             }
         }
         __syncwarp();
-    } else if (warp == 5) {         // ---------------- MMA issuer: per tile P V of the tile before, then the scores
-        bool ok = true;
-        for (int it = 0; ok && it <= n_it; it++) {
-            if (it > 0) {
-                const int j = it - 1, s = j % AT_STAGES;
-                if (!(ok = at_wait(v_full(s), (j / AT_STAGES) & 1, abort_flag))) break;
-                const int nk = last + 1 - (t_lo + j * KT);
-                if (nk < KT) {      // rows behind the sequence's last token are whatever the cache held: zero weights must meet zeros
+    } else if (warp == 5) {         // ---------------- MMA issuer
+        auto scores = [&](int j) {
+            const int s = j % AT_STAGES;
+            if (!at_wait(k_full(s), (j / AT_STAGES) & 1, abort_flag)) return false;
+            tc_fence_after();
+            if (lane == 0) {
+                const uint32_t sk = sm_k + s * Cfg::K_BYTES;
 #pragma unroll
-                    for (int c = 0; c < VP / 64; c++) {
-                        uint4* z = reinterpret_cast<uint4*>(smem + (sm_v - sm_q) + s * Cfg::V_BYTES + c * (KT * 128) + nk * 128);
-                        for (int e = lane; e < (KT - nk) * 8; e += 32) z[e] = make_uint4(0, 0, 0, 0);
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
+                for (int k = 0; k < DP / 16; k++)
+                    umma_f16(tm + (j & 1) * KT, umma_desc_sw128(sm_q + (k >> 2) * (128 * 128) + (k & 3) * 32), umma_desc_sw128(sk + (k >> 2) * (KT * 128) + (k & 3) * 32),
+                             Cfg::IDESC_S, k > 0);
+                umma_commit(k_empty(s));
+                umma_commit(s_bar(j));
+            }
+            __syncwarp();
+            return true;
+        };
+        bool ok = at_wait(q_bar, 0, abort_flag) && scores(0);
+        if (ok && n_it > 1) ok = scores(1);
+        for (int j = 0; ok && j < n_it; j++) {
+            const int s = j % AT_STAGES;
+            if (!(ok = at_wait(v_full(s), (j / AT_STAGES) & 1, abort_flag))) break;
+            const int nk = last + 1 - (t_lo + j * KT);
+            if (nk < KT) {          // rows behind the sequence's last token are whatever the cache held: zero weights must meet zeros
+#pragma unroll
+                for (int c = 0; c < VP / 64; c++) {
+                    uint4* z = reinterpret_cast<uint4*>(smem + (sm_v - sm_q) + s * Cfg::V_BYTES + c * (KT * 128) + nk * 128);
+                    for (int e = lane; e < (KT - nk) * 8; e += 32) z[e] = make_uint4(0, 0, 0, 0);
                 }
-                if (!(ok = at_wait(p_bar, j & 1, abort_flag))) break;
-                tc_fence_after();
-                if (lane == 0) {
-                    const uint32_t sv = sm_v + s * Cfg::V_BYTES;
-#pragma unroll
-                    for (int c = 0; c < VP / 64; c++)
-#pragma unroll
-                        for (int k = 0; k < KT / 16; k++)
-                            umma_f16_ts(tm + Cfg::O_COL + c * 64, tm + Cfg::P_COL + k * 8, umma_desc_sw128(sv + c * (KT * 128) + k * 2048), Cfg::IDESC_O, j > 0 || k > 0);
-                    umma_commit(v_empty(s));
-                    if (it == n_it) umma_commit(o_bar);
-                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
             }
-            if (it < n_it) {
-                const int s = it % AT_STAGES;
-                if (!(ok = at_wait(k_full(s), (it / AT_STAGES) & 1, abort_flag))) break;
-                tc_fence_after();
-                if (lane == 0) {
-                    const uint32_t sk = sm_k + s * Cfg::K_BYTES;
+            if (!(ok = at_wait(p_bar(j), (j >> 1) & 1, abort_flag))) break;
+            tc_fence_after();
+            if (lane == 0) {
+                const uint32_t sv = sm_v + s * Cfg::V_BYTES;
 #pragma unroll
-                    for (int k = 0; k < DP / 16; k++)
-                        umma_f16(tm, umma_desc_sw128(sm_q + (k >> 2) * (128 * 128) + (k & 3) * 32), umma_desc_sw128(sk + (k >> 2) * (KT * 128) + (k & 3) * 32), Cfg::IDESC_S, k > 0);
-                    umma_commit(k_empty(s));
-                    umma_commit(s_bar);          // the scores are there, and the P V before them has read its weights
-                }
-                __syncwarp();
+                for (int c = 0; c < VP / 64; c++)
+#pragma unroll
+                    for (int k = 0; k < KT / 16; k++)
+                        umma_f16_ts(tm + Cfg::O_COL + c * 64, tm + (j & 1) * KT + k * 8, umma_desc_sw128(sv + c * (KT * 128) + k * 2048), Cfg::IDESC_O, j > 0 || k > 0);
+                umma_commit(v_empty(s));
+                umma_commit(o_bar(j));
+            }
+            __syncwarp();
+            if (j + 2 < n_it) {     // the next scores replace the weights that this product reads
+                if (!(ok = at_wait(o_bar(j), (j >> 1) & 1, abort_flag))) break;
+                ok = scores(j + 2);
             }
         }
     } else {                        // ---------------- one row per thread
+        // queries -> bf16, 128-byte swizzle, one 64-column tile after the other; the sign of the scale rides on them
+        const float sgn = a.scale < 0.0f ? -1.0f : 1.0f;
+#pragma unroll
+        for (int e0 = 0; e0 < 128 * (DP / 8); e0 += 128 * 8) {
+            float v[8][8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int e = e0 + i * 128 + threadIdx.x, r = e / (DP / 8), c8 = e % (DP / 8);
+                const float* src = a.Q + (size_t)(row0 + r) * a.ldq + a.q_off + u * DP + c8 * 8;
+                if (r < nq && (((uintptr_t)src) & 15) == 0) {
+                    const float4 x = *reinterpret_cast<const float4*>(src), y = *reinterpret_cast<const float4*>(src + 4);
+                    v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w; v[i][4] = y.x; v[i][5] = y.y; v[i][6] = y.z; v[i][7] = y.w;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) v[i][j] = r < nq ? src[j] : 0.0f;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int e = e0 + i * 128 + threadIdx.x, r = e / (DP / 8), c8 = e % (DP / 8);
+                *reinterpret_cast<uint4*>(smem + (c8 >> 3) * (128 * 128) + r * 128 + (((c8 & 7) ^ (r & 7)) << 4)) =
+                    make_uint4(at_pack(v[i][0] * sgn, v[i][1] * sgn), at_pack(v[i][2] * sgn, v[i][3] * sgn), at_pack(v[i][4] * sgn, v[i][5] * sgn), at_pack(v[i][6] * sgn, v[i][7] * sgn));
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive(q_bar);
+
         const int r = threadIdx.x, pos = pos0 + r;
         const uint32_t tl = tm + ((uint32_t)(warp * 32) << 16);
         const int k_lo = first_key(pos);                                      // this row sees keys k_lo .. pos
@@ -243,11 +268,12 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
         bool ok = true;
         for (int it = 0; it < n_it; it++) {
             const int j0 = t_lo + it * KT;
-            if (!(ok = at_wait(s_bar, it & 1, abort_flag))) break;
+            const uint32_t ts = tl + (it & 1) * KT;
+            if (!(ok = at_wait(s_bar(it), (it >> 1) & 1, abort_flag))) break;
             tc_fence_after();
             float s[KT];
 #pragma unroll
-            for (int c = 0; c < KT / 32; c++) tmem_ld32_nowait(tl + c * 32, s + c * 32);
+            for (int c = 0; c < KT / 32; c++) tmem_ld32_nowait(ts + c * 32, s + c * 32);
             tmem_wait_ld();
             if (!plain) {
 #pragma unroll
@@ -267,15 +293,19 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
                 for (int k = 0; k < KT; k++) s[k] = (k <= hi && k >= lo) ? s[k] : -INFINITY;
             }
             if (!SIG) {
-                float mx0 = s[0], mx1 = s[1], mx2 = s[2], mx3 = s[3];
+                float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-                for (int k = 4; k < KT; k += 4) { mx0 = fmaxf(mx0, s[k]); mx1 = fmaxf(mx1, s[k + 1]); mx2 = fmaxf(mx2, s[k + 2]); mx3 = fmaxf(mx3, s[k + 3]); }
-                const float mn = fmaxf(m, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * sc2);
+                for (int k = 4; k + 8 <= KT; k += 8)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) mx[i] = at_max3(mx[i], s[k + 2 * i], s[k + 2 * i + 1]);
+                const float mn = fmaxf(m, at_max3(at_max3(mx[0], mx[1], mx[2]), mx[3], at_max3(at_max3(s[KT - 4], s[KT - 3], s[KT - 2]), s[KT - 1], s[KT - 1])) * sc2);
                 const bool need = mn - m > 8.0f;
                 if (__any_sync(0xffffffffu, need)) {
                     const float corr = need ? (m == -INFINITY ? 0.0f : at_exp2(m - mn)) : 1.0f;
                     if (need) { m = mn; l *= corr; }
                     if (it > 0) {
+                        if (!(ok = at_wait(o_bar(it - 1), ((it - 1) >> 1) & 1, abort_flag))) break;      // P V of the tile before has to be in O
+                        tc_fence_after();
 #pragma unroll 1
                         for (int c = 0; c < VP; c += 16) {
                             float o[16];
@@ -307,14 +337,14 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
                     }
                     w[j] = at_pack(p0, p1);
                 }
-                tmem_st16(tl + Cfg::P_COL + c / 2, w);
+                tmem_st16(ts + c / 2, w);
             }
             l += l0 + l1;
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive(p_bar);
+            mbar_arrive(p_bar(it));
         }
-        if (ok && (ok = at_wait(o_bar, 0, abort_flag))) {
+        if (ok && (ok = at_wait(o_bar(n_it - 1), ((n_it - 1) >> 1) & 1, abort_flag))) {
             tc_fence_after();
             float f = 1.0f;
             if (!SIG) {
@@ -377,13 +407,13 @@ template <int DP, int VP, bool SIG>
 static int launch(SeqGemmPlan* p, const AttnTc& a, int n_tiles) {
     using Cfg = AtCfg<DP, VP>;
     CUtensorMap tk, tv;
-    int rc = map2d(p, &tk, a.kc, a.cache_rows, a.kv_heads * a.maps * DP, a.ld_k, Cfg::KT);
+    int rc = map2d(p, &tk, a.kc, a.cache_rows, a.kv_heads * a.maps * DP, a.ld_k, AT_KT);
     if (rc) return rc;
-    rc = map2d(p, &tv, a.vc, a.cache_rows, a.kv_heads * VP, a.ld_v, Cfg::KT);
+    rc = map2d(p, &tv, a.vc, a.cache_rows, a.kv_heads * VP, a.ld_v, AT_KT);
     if (rc) return rc;
     static bool attr = false;
     if (!attr) { GTB_CUDA(cudaFuncSetAttribute(k_attn_tc<DP, VP, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM)); attr = true; }
-    k_attn_tc<DP, VP, SIG><<<dim3(n_tiles, a.heads * a.maps), AT_THREADS, Cfg::SMEM, ctx().stream>>>(tk, tv, a, p->d_status);
+    k_attn_tc<DP, VP, SIG><<<dim3(a.heads * a.maps, n_tiles), AT_THREADS, Cfg::SMEM, ctx().stream>>>(tk, tv, a, p->d_status);
     GTB_LAUNCHED();
     return GTB_OK;
 }
