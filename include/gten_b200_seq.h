@@ -237,8 +237,8 @@ int gtb_seq_topk(gtb_seq_t m, int seg, int k, float* h_values, int32_t* h_ids);
 int gtb_seq_last_logits(gtb_seq_t m, int seg, float* h_logits);
 
 /* options: "capture" (1: the residual stream after every layer run of the last pass is kept for gtb_seq_read_capture),
- * "tensor" (1, default: bf16 matrix products of 9 rows or more on tcgen05, routed experts as grouped products from 64 rows on; 0: SIMT
- * kernels only), "tensor_min_rows" (sets both row counts), "graph" (1, default: gtb_seq_decode replays a CUDA graph per step),
+ * "tensor" (1, default: matrix products of 9 rows or more on tcgen05 -- float32 operands as three exact bf16 pieces, fp32 sums --, routed
+ * experts in bf16 mode as grouped products from 64 rows on; 0: SIMT kernels only), "tensor_min_rows" (sets both row counts), "graph" (1, default: gtb_seq_decode replays a CUDA graph per step),
  * "fused_attn" (1, default: tiled kernels of the mixers on prompt portions -- tensor-core attention in bf16 mode, chunked
  * retention and minGRU, chunked mLSTM and delta rule in bf16 mode, expanded keys and values for latent attention; decode rows of latent attention on tensor cores in bf16 mode;
  * 0: the row-at-a-time kernels), "grouped_experts" (1, default: rows sorted by expert and multiplied as groups

@@ -33,3 +33,24 @@ def test_product(M, N, K, accumulate):
     bound = (K + 8) * 2.0 ** -23 * (np.abs(a).astype(np.float64) @ np.abs(w).astype(np.float64).T + np.abs(c0))
     assert got.shape == want.shape
     assert np.all(np.abs(got - want) <= bound)
+
+
+def test_float32_products_on_bf16_pieces():
+    """float32 mode: products of nine rows and more run on three exact bf16 pieces per value; no further from float64 than the FFMA kernels."""
+    from oracle import seq_ref as R
+    from tinyllama_cpp_b200 import reninex
+    seq.init(0)
+    cfg = reninex.make_config(vocab=96, width=160, n_layers=2, ff=416, taps=3, l_heads=4, l_kv=2, l_dim=24, l_vdim=40, r_heads=2, r_dim=32, r_vdim=40, rot_dims=16, loop=(0, 1, 2))
+    desc = reninex.describe(cfg)
+    t = reninex.synth_tensors(desc, 11, gain=1.5)
+    W = {k: R.bf16_to_float(v) for k, v in t.items()}
+    toks = np.random.default_rng(3).integers(0, 96, 300).astype(np.int32)
+    want = R.forward(cfg, W, toks)[0]
+    err = {}
+    for tensor in (1, 0):
+        m = seq.SeqModel(desc, seq.F32, 1, 320, max_rows=128).load(t)           # 300 rows in passes of 128
+        m.set_option("tensor", tensor)
+        got = np.concatenate([m.step([(0, toks[:9])], range(9)), m.step([(0, toks[9:40])], range(31)), m.step([(0, toks[40:])], range(260))])
+        err[tensor] = np.linalg.norm(got - want) / np.linalg.norm(want)
+        m.close()
+    assert err[1] < 1.2 * err[0] + 1e-7, err

@@ -27,6 +27,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <map>
 #include <string>
 #include <vector>
@@ -187,6 +188,8 @@ struct gtb_seq_model {
     void* act = nullptr;                         // expert activations [max_rows * top_max][kfp_max]
     // grouped experts (bf16 mode): rows sorted by expert, groups aligned to 128 rows
     int mpad_max = 0, e_max = 0;
+    bf16* planes = nullptr;                      // fp32 operands cut into three bf16 pieces [planes_rows][3 planes_k]
+    int planes_rows = 0, planes_k = 0;
     bf16 *Xg = nullptr, *actg = nullptr;         // [mpad_max][wp], [mpad_max][kfp_max]
     float *Yg = nullptr, *rw = nullptr;          // [mpad_max][width], [mpad_max]
     int *pair_dst = nullptr, *tile_e = nullptr;  // [max_rows * top_max], [mpad_max / 128]
@@ -299,6 +302,17 @@ int product(gtb_seq_model* m, const void* A, int lda, const bf16* W, int ldw, fl
     if (sizeof(OT) == 2 && m->use_tensor && M >= m->few_rows && m->gp) {
         const int rc = seq_gemm_bf16(m->gp, A, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
         if (rc != -1) return rc;                 // -1: shape not supported by that kernel
+    }
+    if (sizeof(OT) == 4 && m->use_tensor && M >= m->few_rows && m->gp && m->planes && Kp <= m->planes_k && Kp % 64 == 0 && lda % 4 == 0 && ((uintptr_t)A & 15) == 0) {
+        // float32 operands on the bf16 units: three exact pieces per value (see k_split3), in as many rows at a time as the buffer holds
+        int rc = GTB_OK;
+        for (int r0 = 0; r0 < M && rc == GTB_OK; r0 += m->planes_rows) {
+            const int n = std::min(M - r0, m->planes_rows);
+            k_split3<<<n, 256, 0, st>>>(reinterpret_cast<const float*>(A) + (size_t)r0 * lda, lda, Kp, m->planes);
+            GTB_LAUNCHED();
+            rc = seq_gemm_split3(m->gp, m->planes, 3 * Kp, W, ldw, C + (size_t)r0 * ldc, ldc, n, N, Kp, bias, acc);
+        }
+        if (rc != -1) return rc;
     }
     if (M <= 8) {
         if (M <= 1) k_gemv_rows<OT, 1, 4><<<(N + 3) / 4, 256, 0, st>>>(a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
@@ -2207,6 +2221,11 @@ int gtb_seq_create(gtb_seq_t* out, const gtb_seq_config* cfg, const gtb_seq_laye
             TRY(dalloc_t(m, &m->latVx, (size_t)c.n_slots * c.max_ctx * m->lat_vx_max));
         }
     }
+    if (c.mode == GTB_SEQ_F32 || m->ssm_inner_max > 0) {      // (bf16 mode: the scan's step sizes on passes of few rows)
+        m->planes_rows = c.mode == GTB_SEQ_F32 ? m->max_rows : std::min(m->max_rows, 64);
+        m->planes_k = c.mode == GTB_SEQ_F32 ? std::max({wp, m->kout_p_max, m->kfp_max, pad64(2 * W), m->ssm_x_max, m->ssm_dt_max, pad64(m->lat_qr_max)}) : pad64(m->ssm_bc_max);
+        TRY(dalloc_t(m, &m->planes, (size_t)m->planes_rows * 3 * m->planes_k));
+    }
     TRY(dalloc_t(m, &m->logits, R * c.vocab));
     TRY(dalloc(m, &m->opA, R * wp * es));
     TRY(dalloc(m, &m->opB, R * wp * es));
@@ -2222,7 +2241,7 @@ int gtb_seq_create(gtb_seq_t* out, const gtb_seq_config* cfg, const gtb_seq_laye
     TRY(dalloc_t(m, &m->d_slots, c.n_slots));
     m->host_pos.assign(c.n_slots, 0);
     for (int s = 0; s < c.n_slots; s++) TRY(gtb_seq_slot_reset(m, s));
-    if (c.mode == GTB_SEQ_BF16) seq_gemm_create(&m->gp);     // a failure leaves gp null: SIMT kernels only
+    seq_gemm_create(&m->gp);     // a failure leaves gp null: SIMT kernels only
 #undef TRY
 #undef REQ
     GTB_CUDA(cudaStreamSynchronize(ctx().stream));

@@ -57,6 +57,7 @@ struct SqEpi {
     int group_rows;          // rows of W per group
     const float* row_w;      // EPI_RELU2: weight of every row of A; EPI_GEGLU: optional weight of every row
     int act_kind;            // EPI_GEGLU: 0 = gelu_tanh(gate) * up, 1 = silu(gate) * up
+    int w_blocks;            // k-blocks of W: A's k-block kb meets W's kb mod w_blocks (split operands hold several pieces of K one after the other)
 };
 
 // bounded wait: false when the barrier did not complete (or another role gave up)
@@ -145,7 +146,7 @@ k_seq_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                     if (!(ok = sq_wait(bar_empty(s), ph ^ 1, abort_flag))) break;
                     mbar_expect_tx(bar_full(s), Cfg::STAGE_BYTES);
                     const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES;
-                    tma_load_2d(sa, &tmA, bar_full(s), kb * SQ_BK, SWAP ? wrow : arow);
+                    tma_load_2d(sa, &tmA, bar_full(s), (SWAP ? kb % ep.w_blocks : kb) * SQ_BK, SWAP ? wrow : arow);
                     tma_load_2d(sa + Cfg::A_BYTES, &tmB, bar_full(s), kb * SQ_BK, SWAP ? arow : wrow);
                     if (++s == ST) { s = 0; ph ^= 1; }
                 }
@@ -374,7 +375,7 @@ k_seq_skinny(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                 if (!sq_wait(bar_empty(s), ph ^ 1, abort_flag)) break;
                 mbar_expect_tx(bar_full(s), Cfg::STAGE_BYTES);
                 const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES;
-                tma_load_2d(sw, &tmW, bar_full(s), kb * SQ_BK, n0);
+                tma_load_2d(sw, &tmW, bar_full(s), kb % ep.w_blocks * SQ_BK, n0);
                 tma_load_2d(sw + Cfg::W_BYTES, &tmA, bar_full(s), kb * SQ_BK, m0);
                 if (++s == ST) { s = 0; ph ^= 1; }
             }
@@ -575,13 +576,16 @@ static SkChoice skinny_choice(int M, int N, int K) {
     return c;
 }
 
-static int run(SeqGemmPlan* p, int epi, const void* A, int lda, const void* W, int ldw, int M, int N, int K, const SqEpi& ep) {
-    if (!p || K <= 0 || (K % SQ_BK) || (lda % 8) || (ldw % 8) || (((uintptr_t)A | (uintptr_t)W) & 15)) return -1;
+// KW: K of W when A holds several pieces of it (fp32 epilogue only)
+static int run(SeqGemmPlan* p, int epi, const void* A, int lda, const void* W, int ldw, int M, int N, int K, SqEpi ep, int KW = 0) {
+    if (KW == 0) KW = K;
+    if (!p || K <= 0 || (KW % SQ_BK) || (K % KW) || (lda % 8) || (ldw % 8) || (((uintptr_t)A | (uintptr_t)W) & 15)) return -1;
     CUtensorMap ta, tb;
     int rc;
+    ep.w_blocks = KW / SQ_BK;
     const SkChoice sk = skinny_choice(M, N, K);
     if (sk.mt) {
-        rc = make_map(p, &tb, W, N, K, ldw, 128);
+        rc = make_map(p, &tb, W, N, KW, ldw, 128);
         if (rc) return rc;
         rc = make_map(p, &ta, A, M, K, lda, sk.mt);
         if (rc) return rc;
@@ -593,7 +597,7 @@ static int run(SeqGemmPlan* p, int epi, const void* A, int lda, const void* W, i
         // 128-row tiles of A while one wave holds them all (half the MMA rate, but twice the SMs) or no second tile is needed, 256-row tiles
         // beyond (N = 5632, K = 1024, cold: 384 rows 16.3 against 17.7 us, 512 rows 21.2 against 17.8)
         const int bn = M <= 128 || ((M + 127) / 128) * ((N + 127) / 128) <= ctx().sm_count ? 128 : 256;
-        rc = make_map(p, &tb, W, N, K, ldw, SQ_BM);
+        rc = make_map(p, &tb, W, N, KW, ldw, SQ_BM);
         if (rc) return rc;
         rc = make_map(p, &ta, A, M, K, lda, bn);
         if (rc) return rc;
@@ -616,6 +620,12 @@ int seq_gemm_bf16(SeqGemmPlan* p, const void* A, int lda, const void* W, int ldw
     SqEpi ep{};
     ep.C = C; ep.ldc = ldc; ep.bias = bias; ep.accumulate = accumulate; ep.status = p ? p->d_status : nullptr;
     return run(p, SQ_EPI_F32, A, lda, W, ldw, M, N, K, ep);
+}
+
+int seq_gemm_split3(SeqGemmPlan* p, const void* A3, int lda3, const void* W, int ldw, float* C, int ldc, int M, int N, int K, const float* bias, int accumulate) {
+    SqEpi ep{};
+    ep.C = C; ep.ldc = ldc; ep.bias = bias; ep.accumulate = accumulate; ep.status = p ? p->d_status : nullptr;
+    return run(p, SQ_EPI_F32, A3, lda3, W, ldw, M, N, 3 * K, ep, K);
 }
 
 int seq_gemm_bf16_gelu(SeqGemmPlan* p, const void* A, int lda, const void* W, int ldw, void* act, int ld_act, int M, int N, int K) {
