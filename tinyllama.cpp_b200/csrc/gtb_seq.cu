@@ -608,13 +608,29 @@ int run_retention(gtb_seq_model* m, const PassTables& t, int R, int S, const Run
             k_ret_rotate<<<R, 128, 0, st>>>(t, a, m->P, l.n1);
             GTB_LAUNCHED();
         }
-        if (rcfg.smem_kv > 48 * 1024) GTB_CUDA(cudaFuncSetAttribute(k_ret_chunk_kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rcfg.smem_kv));
-        k_ret_chunk_kv<<<dim3(n_chunks, a.heads, nvs), 256, rcfg.smem_kv, st>>>(t, a, m->P, l.n1, S, rcfg.C, rcfg.vs, m->retU);
+        // wide value heads on aligned columns take the kernels with larger register tiles
+        const bool quads = a.dim % 4 == 0 && a.vdim % 4 == 0;
+        const bool wide = quads && rcfg.C == RT_C && a.vdim > 64 && l.n1 % 4 == 0 && (a.q_off | a.k_off | a.v_off) % 4 == 0;
+        const dim3 wgrid(n_chunks, a.heads, (a.vdim + RT_V - 1) / RT_V);
+        if (wide) {
+            constexpr size_t smem = 2 * RT_C * 128 * sizeof(float);
+            GTB_CUDA(cudaFuncSetAttribute(k_ret_kv_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            k_ret_kv_wide<<<wgrid, 256, smem, st>>>(t, a, m->P, l.n1, S, m->retU);
+        } else {
+            if (rcfg.smem_kv > 48 * 1024) GTB_CUDA(cudaFuncSetAttribute(k_ret_chunk_kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rcfg.smem_kv));
+            k_ret_chunk_kv<<<dim3(n_chunks, a.heads, nvs), 256, rcfg.smem_kv, st>>>(t, a, m->P, l.n1, S, rcfg.C, rcfg.vs, m->retU);
+        }
         GTB_LAUNCHED();
-        k_ret_scan<<<dim3(S, a.heads, (a.dim * a.vdim + 255) / 256), 256, 0, st>>>(t, a, S, rcfg.C, m->retU, run.state[bi]);
+        if (quads) k_ret_scan<4><<<dim3(S, a.heads, (a.dim * a.vdim / 4 + 255) / 256), 256, 0, st>>>(t, a, S, rcfg.C, m->retU, run.state[bi]);
+        else k_ret_scan<1><<<dim3(S, a.heads, (a.dim * a.vdim + 255) / 256), 256, 0, st>>>(t, a, S, rcfg.C, m->retU, run.state[bi]);
         GTB_LAUNCHED();
-        if (rcfg.smem_out > 48 * 1024) GTB_CUDA(cudaFuncSetAttribute(k_ret_chunk_out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rcfg.smem_out));
-        k_ret_chunk_out<<<dim3(n_chunks, a.heads, nvs), 256, rcfg.smem_out, st>>>(t, a, m->P, l.n1, S, rcfg.C, rcfg.vs, m->retU, m->O);
+        if (wide) {
+            GTB_CUDA(cudaFuncSetAttribute(k_ret_out_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RT_OUT_SMEM));
+            k_ret_out_wide<<<wgrid, 256, RT_OUT_SMEM, st>>>(t, a, m->P, l.n1, S, m->retU, m->O);
+        } else {
+            if (rcfg.smem_out > 48 * 1024) GTB_CUDA(cudaFuncSetAttribute(k_ret_chunk_out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rcfg.smem_out));
+            k_ret_chunk_out<<<dim3(n_chunks, a.heads, nvs), 256, rcfg.smem_out, st>>>(t, a, m->P, l.n1, S, rcfg.C, rcfg.vs, m->retU, m->O);
+        }
         GTB_LAUNCHED();
         return post();
     }

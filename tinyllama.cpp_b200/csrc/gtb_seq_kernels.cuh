@@ -806,34 +806,48 @@ __global__ void __launch_bounds__(256) k_ret_chunk_kv(PassTables t, RetBranch b,
     }
 }
 
-// grid (segments, heads, blocks of state elements): every state element walks the segment's chunks on its own
+template <int V> __device__ __forceinline__ void rs_load(const float* p, float (&v)[V]) {
+    if (V == 4) { const float4 x = *reinterpret_cast<const float4*>(p); v[0] = x.x; v[V > 1 ? 1 : 0] = x.y; v[V > 2 ? 2 : 0] = x.z; v[V > 3 ? 3 : 0] = x.w; }
+    else v[0] = *p;
+}
+template <int V> __device__ __forceinline__ void rs_store(float* p, const float (&v)[V]) {
+    if (V == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[V > 1 ? 1 : 0], v[V > 2 ? 2 : 0], v[V > 3 ? 3 : 0]);
+    else *p = v[0];
+}
+// grid (segments, heads, blocks of state elements): V neighbouring state elements (4 where the state's size allows) walk the segment's chunks
+// on their own; a batch's loads are issued before the dependent chain of multiply-adds starts
+template <int V>
 __global__ void __launch_bounds__(256) k_ret_scan(PassTables t, RetBranch b, int S, int C, float* __restrict__ U, float* __restrict__ state) {
+    constexpr int NB = V == 4 ? 8 : 16;
     const int seg = blockIdx.x, h = blockIdx.y;
-    const int e = blockIdx.z * blockDim.x + threadIdx.x;
+    const int e = (blockIdx.z * blockDim.x + threadIdx.x) * V;
     if (e >= b.dim * b.vdim) return;
     int first = 0;
     for (int s = 0; s < seg; s++) first += (t.seg_len[s] + C - 1) / C;
     const int len = t.seg_len[seg], nchunk = (len + C - 1) / C, slot = t.seg_slot[seg];
-    float* gs = state + ((size_t)slot * b.heads + h) * (size_t)b.dim * b.vdim;
+    float* gs = state + ((size_t)slot * b.heads + h) * (size_t)b.dim * b.vdim + e;
     const float lg = logf(b.decay[h]);
     const float gc = expf(lg * (float)C);
-    float s0 = gs[e];
+    float s0[V];
+    rs_load<V>(gs, s0);
     float* u = U + (((size_t)first * b.heads + h) * b.dim) * b.vdim + e;
     const size_t stride = (size_t)b.heads * b.dim * b.vdim;
-    // batches of 16 chunks: all of a batch's loads are issued before the dependent chain of multiply-adds starts
-    for (int c0 = 0; c0 < nchunk; c0 += 16) {
-        float add[16];
+    for (int c0 = 0; c0 < nchunk; c0 += NB) {
+        float add[NB][V];
 #pragma unroll
-        for (int i = 0; i < 16; i++) add[i] = (c0 + i < nchunk) ? u[(size_t)(c0 + i) * stride] : 0.0f;
+        for (int i = 0; i < NB; i++)
+            if (c0 + i < nchunk) rs_load<V>(u + (size_t)(c0 + i) * stride, add[i]);
 #pragma unroll
-        for (int i = 0; i < 16; i++)
+        for (int i = 0; i < NB; i++)
             if (c0 + i < nchunk) {
-                u[(size_t)(c0 + i) * stride] = s0;
+                rs_store<V>(u + (size_t)(c0 + i) * stride, s0);
                 const int Lc = min(C, len - (c0 + i) * C);
-                s0 = fmaf(Lc == C ? gc : expf(lg * (float)Lc), s0, add[i]);
+                const float g = Lc == C ? gc : expf(lg * (float)Lc);
+#pragma unroll
+                for (int j = 0; j < V; j++) s0[j] = fmaf(g, s0[j], add[i][j]);
             }
     }
-    if (!t.slots[slot].stopped) gs[e] = s0;
+    if (!t.slots[slot].stopped) rs_store<V>(gs, s0);
 }
 
 // grid (chunks, heads, value slices); Sb [chunk][head][dim][vdim] = state before the chunk; O [R][heads * vdim].
@@ -931,6 +945,209 @@ __global__ void __launch_bounds__(256) k_ret_chunk_out(PassTables t, RetBranch b
 #pragma unroll
             for (int y = 0; y < 4; y++)
                 if (j4 + y < nv) O[(size_t)(row0 + a4 + x) * (b.heads * b.vdim) + h * b.vdim + j0 + j4 + y] = fmaf(ga, inter[x][y], intra[x][y]);
+        }
+    }
+}
+
+// The same two kernels for value heads of more than 64 and up to 128 channels per slice (heads of at most 128, everything a multiple of four and
+// 16-byte aligned): register tiles of 8 x 8 and 4 x 8 on packed fp32 multiply-adds, so that the shared-memory reads of a step are a small
+// part of its arithmetic, and scores once per chunk and head.  Same sums in the same precision.  Bound: the FFMA rate (2048 rows, 16 heads
+// of 128 | 128: 15 and 22 us of multiply-adds).
+__device__ __forceinline__ uint64_t rt_pair(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 rt_split(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void rt_fma2(uint64_t& d, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+constexpr int RT_C = 64, RT_V = 128;      // rows per chunk, value channels per slice
+
+// U [chunk][head][dim][vdim]; grid (chunks, heads, value slices), 256 threads.  Shared memory: k' [64][128], v [64][128] (zeros beyond the head)
+__global__ void __launch_bounds__(256) k_ret_kv_wide(PassTables t, RetBranch b, const float* __restrict__ P, int ldp, int S, float* __restrict__ U) {
+    extern __shared__ __align__(16) float sm[];
+    float* sk = sm;
+    float* sv = sm + RT_C * 128;
+    int seg, c;
+    if (!ret_find_chunk(t, S, RT_C, blockIdx.x, seg, c)) return;
+    const int h = blockIdx.y, j0 = blockIdx.z * RT_V, nv = min(RT_V, b.vdim - j0);
+    const int row0 = t.seg_row0[seg] + c * RT_C, L = min(RT_C, t.seg_len[seg] - c * RT_C);
+    const float lg = logf(b.decay[h]);
+    const int i4 = (threadIdx.x & 31) * 4, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int p = 0; p < RT_C / 8; p++) {
+        const int bb = p * 8 + w;
+        float4 k = make_float4(0, 0, 0, 0), v = k;
+        if (bb < L) {
+            const float* row = P + (size_t)(row0 + bb) * ldp;
+            if (i4 < b.dim) k = *reinterpret_cast<const float4*>(row + b.k_off + h * b.dim + i4);
+            if (i4 < nv) v = *reinterpret_cast<const float4*>(row + b.v_off + h * b.vdim + j0 + i4);
+        }
+        const float g = expf(lg * (float)(L - 1 - bb));
+        *reinterpret_cast<float4*>(sk + bb * 128 + i4) = bb < L ? make_float4(k.x * g, k.y * g, k.z * g, k.w * g) : k;
+        *reinterpret_cast<float4*>(sv + bb * 128 + i4) = v;
+    }
+    __syncthreads();
+    const int tj = threadIdx.x & 15, ti = threadIdx.x >> 4;            // rows 4 ti .. + 3 and 64 + 4 ti .. + 3, columns likewise
+    uint64_t acc[8][4] = {};
+#pragma unroll 2
+    for (int bb = 0; bb < L; bb++) {
+        const float4 ka = *reinterpret_cast<const float4*>(sk + bb * 128 + 4 * ti), kb = *reinterpret_cast<const float4*>(sk + bb * 128 + 64 + 4 * ti);
+        const float4 va = *reinterpret_cast<const float4*>(sv + bb * 128 + 4 * tj), vb = *reinterpret_cast<const float4*>(sv + bb * 128 + 64 + 4 * tj);
+        const uint64_t v2[4] = {rt_pair(va.x, va.y), rt_pair(va.z, va.w), rt_pair(vb.x, vb.y), rt_pair(vb.z, vb.w)};
+        const float kk[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+#pragma unroll
+        for (int x = 0; x < 8; x++) {
+            const uint64_t k2 = rt_pair(kk[x], kk[x]);
+#pragma unroll
+            for (int y = 0; y < 4; y++) rt_fma2(acc[x][y], k2, v2[y]);
+        }
+    }
+    float* u = U + (((size_t)blockIdx.x * b.heads + h) * b.dim) * b.vdim + j0;
+#pragma unroll
+    for (int x = 0; x < 8; x++) {
+        const int i = (x >> 2) * 64 + 4 * ti + (x & 3);
+        if (i >= b.dim) continue;
+#pragma unroll
+        for (int y = 0; y < 2; y++) {
+            const int j = y * 64 + 4 * tj;
+            const float2 lo = rt_split(acc[x][2 * y]), hi = rt_split(acc[x][2 * y + 1]);
+            if (j < nv) *reinterpret_cast<float4*>(u + (size_t)i * b.vdim + j) = make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+    }
+}
+
+// O [R][heads * vdim]; grid (chunks, heads, value slices), 256 threads.  o_a = g^(a+1) sum_i q_a[i] S0[i] + sum_{b <= a} g^(a-b) (q_a . k_b) v_b: the
+// scores first (4 x 4 tiles), then one product over the 128-row state and the chunk's 64 values, streamed in tiles of 32 rows through
+// the space of the keys.  Shared memory: qT [128][68], kT [128][68] / two tiles [32][128], weights aT [64 keys][64 rows]
+constexpr int RT_CP = RT_C + 4;
+constexpr size_t RT_OUT_SMEM = (2 * 128 * RT_CP + RT_C * RT_C + RT_C + 4) * sizeof(float);
+__global__ void __launch_bounds__(256, 2) k_ret_out_wide(PassTables t, RetBranch b, const float* __restrict__ P, int ldp, int S, const float* __restrict__ Sb, float* __restrict__ O) {
+    extern __shared__ __align__(16) float sm[];
+    float* sq = sm;                        // [128][RT_CP]
+    float* sk = sq + 128 * RT_CP;          // [128][RT_CP]; then [2][32][128]
+    float* sa = sk + 128 * RT_CP;          // [64][64]
+    float* pw = sa + RT_C * RT_C;          // decay powers 0 .. 64
+    int seg, c;
+    if (!ret_find_chunk(t, S, RT_C, blockIdx.x, seg, c)) return;
+    const int h = blockIdx.y, j0 = blockIdx.z * RT_V, nv = min(RT_V, b.vdim - j0);
+    const int row0 = t.seg_row0[seg] + c * RT_C, L = min(RT_C, t.seg_len[seg] - c * RT_C);
+    const float lg = logf(b.decay[h]);
+    if (threadIdx.x <= RT_C) pw[threadIdx.x] = expf(lg * (float)threadIdx.x);
+    // queries and keys, transposed: a quarter warp reads 64 contiguous bytes of two rows
+    {
+        const int rr = (threadIdx.x >> 2) & 63, c4 = (threadIdx.x & 3) * 4;
+        const float* row = P + (size_t)(row0 + rr) * ldp;
+        float4 q[8], k[8];
+#pragma unroll
+        for (int x = 0; x < 8; x++) {
+            const int i = x * 16 + c4;
+            const bool in = rr < L && i < b.dim;
+            q[x] = in ? *reinterpret_cast<const float4*>(row + b.q_off + h * b.dim + i) : make_float4(0, 0, 0, 0);
+            k[x] = in ? *reinterpret_cast<const float4*>(row + b.k_off + h * b.dim + i) : make_float4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int x = 0; x < 8; x++) {
+            const int i = x * 16 + c4;
+            sq[i * RT_CP + rr] = q[x].x; sq[(i + 1) * RT_CP + rr] = q[x].y; sq[(i + 2) * RT_CP + rr] = q[x].z; sq[(i + 3) * RT_CP + rr] = q[x].w;
+            sk[i * RT_CP + rr] = k[x].x; sk[(i + 1) * RT_CP + rr] = k[x].y; sk[(i + 2) * RT_CP + rr] = k[x].z; sk[(i + 3) * RT_CP + rr] = k[x].w;
+        }
+    }
+    __syncthreads();
+    {
+        const int a4 = (threadIdx.x >> 4) * 4, b4 = (threadIdx.x & 15) * 4;
+        uint64_t acc[4][2] = {};                          // [key][rows in pairs]
+        if (b4 <= a4 + 3 && a4 < L) {
+#pragma unroll 4
+            for (int i = 0; i < b.dim; i++) {
+                const float4 q4 = *reinterpret_cast<const float4*>(sq + i * RT_CP + a4), k4 = *reinterpret_cast<const float4*>(sk + i * RT_CP + b4);
+                const uint64_t q2[2] = {rt_pair(q4.x, q4.y), rt_pair(q4.z, q4.w)};
+                const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+                for (int y = 0; y < 4; y++) {
+                    const uint64_t k2 = rt_pair(kk[y], kk[y]);
+                    rt_fma2(acc[y][0], k2, q2[0]);
+                    rt_fma2(acc[y][1], k2, q2[1]);
+                }
+            }
+        }
+#pragma unroll
+        for (int y = 0; y < 4; y++) {
+            const int bb = b4 + y;
+            const float2 lo = rt_split(acc[y][0]), hi = rt_split(acc[y][1]);
+            const float v[4] = {lo.x, lo.y, hi.x, hi.y};
+            float o[4];
+#pragma unroll
+            for (int x = 0; x < 4; x++) o[x] = bb <= a4 + x ? v[x] * pw[a4 + x - bb] : 0.0f;
+            *reinterpret_cast<float4*>(sa + bb * RT_C + a4) = make_float4(o[0], o[1], o[2], o[3]);
+        }
+    }
+    __syncthreads();
+    // tiles of 32 rows: the state's (dim rounded up to 32), then the values'
+    const float* sb = Sb + (((size_t)blockIdx.x * b.heads + h) * b.dim) * b.vdim + j0;
+    const int n_st = (b.dim + 31) / 32, n_t = n_st + (L + 31) / 32;
+    auto load = [&](int it) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(sk + (it & 1) * (32 * RT_V));
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+            const int rr = (threadIdx.x >> 5) + x * 8, j = (threadIdx.x & 31) * 4;
+            const int i = (it < n_st ? it : it - n_st) * 32 + rr;
+            const bool ok = j < nv && i < (it < n_st ? b.dim : L);
+            const float* src = it < n_st ? sb + (size_t)i * b.vdim + j : P + (size_t)(row0 + i) * ldp + b.v_off + h * b.vdim + j0 + j;
+            const int n = ok ? 16 : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)((rr * RT_V + j) * 4)), "l"(ok ? src : sb), "r"(n) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int a4 = (threadIdx.x >> 4) * 4, tj = threadIdx.x & 15;      // rows a4 .. + 3, columns 4 tj .. + 3 and 64 + 4 tj .. + 3
+    uint64_t acc[4][4] = {};
+    load(0);
+    for (int it = 0; it < n_t; it++) {
+        if (it + 1 < n_t) { load(it + 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (it == n_st) {                                  // the state's share carries the decay since the chunk's start
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                const uint64_t g2 = rt_pair(pw[a4 + x + 1], pw[a4 + x + 1]);
+#pragma unroll
+                for (int y = 0; y < 4; y++) {
+                    const float2 v = rt_split(acc[x][y]), g = rt_split(g2);
+                    acc[x][y] = rt_pair(v.x * g.x, v.y * g.y);
+                }
+            }
+        }
+        const float* tile = sk + (it & 1) * (32 * RT_V);
+        const float* left = it < n_st ? sq + it * 32 * RT_CP + a4 : sa + (it - n_st) * 32 * RT_C + a4;
+        const int ldl = it < n_st ? RT_CP : RT_C;
+        const int n = it < n_st ? 32 : min(32, a4 + 4 - (it - n_st) * 32);      // (weights behind a row's position are zeros)
+#pragma unroll 4
+        for (int i = 0; i < n; i++) {
+            const float4 l4 = *reinterpret_cast<const float4*>(left + i * ldl);
+            const float4 va = *reinterpret_cast<const float4*>(tile + i * RT_V + 4 * tj), vb = *reinterpret_cast<const float4*>(tile + i * RT_V + 64 + 4 * tj);
+            const uint64_t v2[4] = {rt_pair(va.x, va.y), rt_pair(va.z, va.w), rt_pair(vb.x, vb.y), rt_pair(vb.z, vb.w)};
+            const float ll[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                const uint64_t l2 = rt_pair(ll[x], ll[x]);
+#pragma unroll
+                for (int y = 0; y < 4; y++) rt_fma2(acc[x][y], l2, v2[y]);
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+        if (a4 + x >= L) continue;
+        float* o = O + (size_t)(row0 + a4 + x) * (b.heads * b.vdim) + h * b.vdim + j0;
+#pragma unroll
+        for (int y = 0; y < 2; y++) {
+            const int j = y * 64 + 4 * tj;
+            const float2 lo = rt_split(acc[x][2 * y]), hi = rt_split(acc[x][2 * y + 1]);
+            if (j < nv) *reinterpret_cast<float4*>(o + j) = make_float4(lo.x, lo.y, hi.x, hi.y);
         }
     }
 }
