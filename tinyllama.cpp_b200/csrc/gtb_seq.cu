@@ -308,20 +308,20 @@ int product(gtb_seq_model* m, const void* A, int lda, const bf16* W, int ldw, fl
         int rc = GTB_OK;
         for (int r0 = 0; r0 < M && rc == GTB_OK; r0 += m->planes_rows) {
             const int n = std::min(M - r0, m->planes_rows);
-            k_split3<<<n, 256, 0, st>>>(reinterpret_cast<const float*>(A) + (size_t)r0 * lda, lda, Kp, m->planes);
+            pdl_launch(k_split3, n, 256, 0, st, reinterpret_cast<const float*>(A) + (size_t)r0 * lda, lda, Kp, m->planes);
             GTB_LAUNCHED();
             rc = seq_gemm_split3(m->gp, m->planes, 3 * Kp, W, ldw, C + (size_t)r0 * ldc, ldc, n, N, Kp, bias, acc);
         }
         if (rc != -1) return rc;
     }
     if (M <= 8) {
-        if (M <= 1) k_gemv_rows<OT, 1, 4><<<(N + 3) / 4, 256, 0, st>>>(a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
-        else if (M <= 2) k_gemv_rows<OT, 2, 4><<<(N + 3) / 4, 256, 0, st>>>(a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
-        else if (M <= 4) k_gemv_rows<OT, 4, 4><<<(N + 3) / 4, 256, 0, st>>>(a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
-        else k_gemv_rows<OT, 8, 4><<<(N + 3) / 4, 256, 0, st>>>(a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
+        if (M <= 1) pdl_launch(k_gemv_rows<OT, 1, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
+        else if (M <= 2) pdl_launch(k_gemv_rows<OT, 2, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
+        else if (M <= 4) pdl_launch(k_gemv_rows<OT, 4, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
+        else pdl_launch(k_gemv_rows<OT, 8, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
     } else {
         dim3 grid((N + SG_BN - 1) / SG_BN, (M + SG_BM - 1) / SG_BM);
-        k_gemm_simt<OT><<<grid, 256, 0, st>>>(a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
+        pdl_launch(k_gemm_simt<OT>, grid, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
     }
     GTB_LAUNCHED();
     return GTB_OK;
@@ -360,7 +360,7 @@ int launch_sigattn_mma(const PassTables& t, const AttnBranch& a, int S, int n_ti
     const size_t smem = ((HPC + 2) * 64 * (size_t)(DP + 8) + 2 * 64 * (size_t)(VP + 8)) * 2;      // queries + two stages of keys and values
     static bool attr = false;
     if (!attr) { GTB_CUDA(cudaFuncSetAttribute(k_sigattn_mma<DP, VP, HPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr = true; }
-    k_sigattn_mma<DP, VP, HPC><<<dim3(n_tiles, a.heads / HPC), 128 * HPC, smem, ctx().stream>>>(t, a, S, P, ldp, kc, vc, out, ld_out);
+    pdl_launch(k_sigattn_mma<DP, VP, HPC>, dim3(n_tiles, a.heads / HPC), 128 * HPC, smem, ctx().stream, t, a, S, P, ldp, kc, vc, out, ld_out);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -407,7 +407,7 @@ int launch_sattn_mma(const PassTables& t, const SoftAttn& a, int S, int n_tiles,
     const size_t smem = (3 * 64 * (size_t)(DP + 8) + 2 * 64 * (size_t)(VP + 8)) * 2;      // queries + two stages of keys and values
     static bool attr = false;
     if (!attr) { GTB_CUDA(cudaFuncSetAttribute(k_sattn_mma<DP, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr = true; }
-    k_sattn_mma<DP, VP><<<dim3(n_tiles, a.heads * sa_maps(a)), 128, smem, ctx().stream>>>(t, a, S, P, ldp, kc, vc, pk, pv, out, ld_out, out_f, ld_f);
+    pdl_launch(k_sattn_mma<DP, VP>, dim3(n_tiles, a.heads * sa_maps(a)), 128, smem, ctx().stream, t, a, S, P, ldp, kc, vc, pk, pv, out, ld_out, out_f, ld_f);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -461,7 +461,7 @@ int run_postnorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
     const int W = c.width, wp = m->wp;
     OT *opA = (OT*)m->opA, *opC = (OT*)m->opC;
     if (!x_in_opA) {
-        k_copy_operand<OT><<<R, 256, 0, st>>>(m->x, W, opA, (OT*)nullptr, wp);
+        pdl_launch(k_copy_operand<OT>, R, 256, 0, st, m->x, W, opA, (OT*)nullptr, wp);
         GTB_LAUNCHED();
     }
     int rc = product<OT>(m, opA, wp, l.w_mix, wp, m->P, l.n1, R, l.n1, wp, l.d_bias, 0);
@@ -474,22 +474,22 @@ int run_postnorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
             int n_chunks = 0;
             for (int s = 0; s < S; s++) n_chunks += (seg_lens[s] + GRU_CHUNK - 1) / GRU_CHUNK;
             if ((size_t)n_chunks * 2 * a.width > m->gruAB_floats) return gtb::fail(GTB_ERR_STATE, "chunk workspace too small");
-            k_mingru_chunk<<<dim3(n_chunks, cb), 128, 0, st>>>(t, a, m->P, l.n1, S, GRU_CHUNK, m->gruAB);
+            pdl_launch(k_mingru_chunk, dim3(n_chunks, cb), 128, 0, st, t, a, m->P, l.n1, S, GRU_CHUNK, m->gruAB);
             GTB_LAUNCHED();
-            k_mingru_chunk_out<OT><<<dim3(n_chunks, cb), 128, 0, st>>>(t, a, m->P, l.n1, S, GRU_CHUNK, m->gruAB, run.state[0], opC, l.kout_p);
+            pdl_launch(k_mingru_chunk_out<OT>, dim3(n_chunks, cb), 128, 0, st, t, a, m->P, l.n1, S, GRU_CHUNK, m->gruAB, run.state[0], opC, l.kout_p);
             GTB_LAUNCHED();
-            k_mingru_store<<<dim3(S, cb), 128, 0, st>>>(t, a, S, GRU_CHUNK, m->gruAB, run.state[0]);
+            pdl_launch(k_mingru_store, dim3(S, cb), 128, 0, st, t, a, S, GRU_CHUNK, m->gruAB, run.state[0]);
             GTB_LAUNCHED();
         } else {
-            k_mingru<OT><<<dim3(S, cb), 128, 0, st>>>(t, a, m->P, l.n1, run.state[0], opC, l.kout_p);
+            pdl_launch(k_mingru<OT>, dim3(S, cb), 128, 0, st, t, a, m->P, l.n1, run.state[0], opC, l.kout_p);
             GTB_LAUNCHED();
         }
     } else {
         const SoftAttn a = soft_args(m, b, run);
-        k_sattn_prep<OT><<<dim3(R, (a.heads + 2 * a.kv_heads + 3) / 4), 128, 0, st>>>(t, a, m->P, l.n1, (OT*)run.kc[0], (OT*)run.vc[0]);
+        pdl_launch(k_sattn_prep<OT>, dim3(R, (a.heads + 2 * a.kv_heads + 3) / 4), 128, 0, st, t, a, m->P, l.n1, (OT*)run.kc[0], (OT*)run.vc[0]);
         GTB_LAUNCHED();
         if (a.pool > 0) {
-            k_pool_update<OT><<<R, 128, 0, st>>>(t, a, (const OT*)run.kc[0], (const OT*)run.vc[0], run.pk, run.pv);
+            pdl_launch(k_pool_update<OT>, R, 128, 0, st, t, a, (const OT*)run.kc[0], (const OT*)run.vc[0], run.pk, run.pv);
             GTB_LAUNCHED();
         }
         int done = -1;
@@ -501,15 +501,15 @@ int run_postnorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
             const int max_keys = a.window > 0 ? std::min(c.max_ctx, a.window + (a.pool > 0 ? c.max_ctx / a.pool : 0)) : c.max_ctx;
             const int splits = std::max(1, std::min(32, (max_keys + 127) / 128));
             if (splits > 1) {
-                k_sattn_split<OT><<<dim3(R, a.heads, splits), 128, (a.dim + 128 + 33) * sizeof(float), st>>>(t, a, m->P, l.n1, (const OT*)run.kc[0], (const OT*)run.vc[0], run.pk, run.pv, m->sattn_part, R);
+                pdl_launch(k_sattn_split<OT>, dim3(R, a.heads, splits), 128, (a.dim + 128 + 33) * sizeof(float), st, t, a, m->P, l.n1, (const OT*)run.kc[0], (const OT*)run.vc[0], run.pk, run.pv, m->sattn_part, R);
                 GTB_LAUNCHED();
-                k_sattn_join<OT><<<dim3(R, a.heads), 128, 0, st>>>(a, m->P, l.n1, m->sattn_part, R, splits, opC, l.kout_p);
+                pdl_launch(k_sattn_join<OT>, dim3(R, a.heads), 128, 0, st, a, m->P, l.n1, m->sattn_part, R, splits, opC, l.kout_p);
                 GTB_LAUNCHED();
                 done = 0;
             }
         }
         if (done < 0) {
-            k_sattn<OT><<<dim3(R, a.heads), 128, (a.dim + 128 + 33) * sizeof(float), st>>>(t, a, m->P, l.n1, (const OT*)run.kc[0], (const OT*)run.vc[0], run.pk, run.pv, opC, l.kout_p);
+            pdl_launch(k_sattn<OT>, dim3(R, a.heads), 128, (a.dim + 128 + 33) * sizeof(float), st, t, a, m->P, l.n1, (const OT*)run.kc[0], (const OT*)run.vc[0], run.pk, run.pv, opC, l.kout_p);
             GTB_LAUNCHED();
         }
     }
@@ -521,17 +521,17 @@ int run_postnorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
     const bool routed = l.ff > 0 && l.d.ff_kind == GTB_FF_EXPERTS;
     const size_t rn_smem = routed ? ((size_t)W + 3 * l.n_out) * sizeof(float) : 0;
     if (routed && R <= 8 && rn_smem <= 40 * 1024) { rn.w = l.w_router; rn.ldw = wp; rn.n_out = l.n_out; rn.top = l.d.top; rn.corr = l.d_corr; rn.sel_idx = m->sel_idx; rn.sel_w = m->sel_w; }
-    k_postnorm_add<OT><<<R, 256, rn.w ? rn_smem : 0, st>>>(m->Y, W, c.eps, l.norm1, nullptr, nullptr, 0, 0, nullptr, nullptr, m->x, opA, wp, rn);
+    pdl_launch(k_postnorm_add<OT>, R, 256, rn.w ? rn_smem : 0, st, m->Y, W, c.eps, l.norm1, nullptr, nullptr, 0, 0, nullptr, nullptr, m->x, opA, wp, rn);
     GTB_LAUNCHED();
     if (l.ff == 0) return GTB_OK;
     if (l.d.ff_kind == GTB_FF_POLYNORM) {
         rc = product<OT>(m, opA, wp, l.w_up, wp, m->G, l.ff, R, l.ff, wp, nullptr, 0);
         if (rc) return rc;
-        k_polynorm<OT><<<R, 256, 0, st>>>(m->G, l.ff, l.ff, c.eps, l.d_act, opC, l.kfp);
+        pdl_launch(k_polynorm<OT>, R, 256, 0, st, m->G, l.ff, l.ff, c.eps, l.d_act, opC, l.kfp);
         GTB_LAUNCHED();
         rc = product<OT>(m, opC, l.kfp, l.w_down, l.kfp, m->Y, W, R, W, l.kfp, nullptr, 0);
         if (rc) return rc;
-        k_postnorm_add<OT><<<R, 256, 0, st>>>(m->Y, W, c.eps, l.norm2, nullptr, nullptr, 0, 0, nullptr, nullptr, m->x, opA, wp, RouteNext{});
+        pdl_launch(k_postnorm_add<OT>, R, 256, 0, st, m->Y, W, c.eps, l.norm2, nullptr, nullptr, 0, 0, nullptr, nullptr, m->x, opA, wp, RouteNext{});
         GTB_LAUNCHED();
         return GTB_OK;
     }
@@ -539,22 +539,22 @@ int run_postnorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
     if (!rn.w) {
         rc = product<OT>(m, opA, wp, l.w_router, wp, m->rl, l.n_out, R, l.n_out, wp, nullptr, 0);
         if (rc) return rc;
-        k_moe_route<<<R, 32, 2 * l.n_out * sizeof(float), st>>>(m->rl, l.n_out, l.n_out, l.d_corr, top, m->sel_idx, m->sel_w);
+        pdl_launch(k_moe_route, R, 32, 2 * l.n_out * sizeof(float), st, m->rl, l.n_out, l.n_out, l.d_corr, top, m->sel_idx, m->sel_w);
         GTB_LAUNCHED();
     }
     const int n_pairs = R * top, mpad = (n_pairs + 127) / 128 * 128 + E * 128;
     if (sizeof(OT) == 2 && E > 0 && m->grouped_experts && m->use_tensor && m->gp && m->Xg && R >= m->tensor_min_rows && mpad <= m->mpad_max) {
         // rows sorted by expert, two grouped tensor-core products (up with the weighted relu^2 epilogue, down), the choices of a row summed
         // in the residual update
-        k_moe_group<<<1, 1024, 2 * E * sizeof(int), st>>>(m->sel_idx, n_pairs, E, m->pair_dst, m->tile_e, mpad / 128);
+        pdl_launch(k_moe_group, 1, 1024, 2 * E * sizeof(int), st, m->sel_idx, n_pairs, E, m->pair_dst, m->tile_e, mpad / 128);
         GTB_LAUNCHED();
-        k_moe_gather<<<n_pairs, 128, 0, st>>>((const bf16*)opA, wp, top, m->pair_dst, m->sel_w, m->Xg, m->rw);
+        pdl_launch(k_moe_gather, n_pairs, 128, 0, st, (const bf16*)opA, wp, top, m->pair_dst, m->sel_w, m->Xg, m->rw);
         GTB_LAUNCHED();
         rc = seq_gemm_bf16_grouped(m->gp, m->Xg, wp, l.w_up, wp, mpad, l.ff, wp, E, m->tile_e, nullptr, 0, m->actg, l.kfp, m->rw);
         if (rc == 0) rc = seq_gemm_bf16_grouped(m->gp, m->actg, l.kfp, l.w_down, l.kfp, mpad, W, l.kfp, E, m->tile_e, m->Yg, W, nullptr, 0, nullptr);
         if (rc > 0) return rc;
         if (rc == 0) {
-            k_postnorm_add<OT><<<R, 256, 0, st>>>(nullptr, W, c.eps, l.norm2, m->sel_idx, m->sel_w, top, E, m->Yg, m->pair_dst, m->x, opA, wp, RouteNext{});
+            pdl_launch(k_postnorm_add<OT>, R, 256, 0, st, nullptr, W, c.eps, l.norm2, m->sel_idx, m->sel_w, top, E, m->Yg, m->pair_dst, m->x, opA, wp, RouteNext{});
             GTB_LAUNCHED();
             return GTB_OK;
         }
@@ -563,14 +563,14 @@ int run_postnorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
         // a warp per output column; with few (row, choice) pairs every column group gets its own CTA so that the experts' matrices stream at
         // full width, with many pairs the grid is wide already
         const int cta_budget = std::max(1, 4096 / std::max(1, R * top));
-        k_moe_up_rows<OT><<<dim3(R * top, std::max(1, std::min(cta_budget, (l.kfp + 7) / 8))), 256, 0, st>>>(opA, wp, wp, l.w_up, wp, l.ff, l.kfp, E, top, m->sel_idx, m->sel_w, (OT*)m->act);
+        pdl_launch(k_moe_up_rows<OT>, dim3(R * top, std::max(1, std::min(cta_budget, (l.kfp + 7) / 8))), 256, 0, st, opA, wp, wp, l.w_up, wp, l.ff, l.kfp, E, top, m->sel_idx, m->sel_w, (OT*)m->act);
         GTB_LAUNCHED();
-        k_moe_down_rows<OT><<<dim3(R, std::max(1, std::min(std::max(1, 4096 / R), (W + 7) / 8))), 256, 0, st>>>((const OT*)m->act, l.kfp, l.w_down, W, E, top, m->sel_idx, m->Y, W);
+        pdl_launch(k_moe_down_rows<OT>, dim3(R, std::max(1, std::min(std::max(1, 4096 / R), (W + 7) / 8))), 256, 0, st, (const OT*)m->act, l.kfp, l.w_down, W, E, top, m->sel_idx, m->Y, W);
         GTB_LAUNCHED();
     } else {
         GTB_CUDA(cudaMemsetAsync(m->Y, 0, (size_t)R * W * sizeof(float), st));
     }
-    k_postnorm_add<OT><<<R, 256, 0, st>>>(m->Y, W, c.eps, l.norm2, m->sel_idx, m->sel_w, top, E, nullptr, nullptr, m->x, opA, wp, RouteNext{});
+    pdl_launch(k_postnorm_add<OT>, R, 256, 0, st, m->Y, W, c.eps, l.norm2, m->sel_idx, m->sel_w, top, E, nullptr, nullptr, m->x, opA, wp, RouteNext{});
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -589,12 +589,12 @@ int run_retention(gtb_seq_model* m, const PassTables& t, int R, int S, const Run
         // in place, in one pass over q | k | v (neighbours in the projection): activating inside the chunk kernels instead was measured
         // slower (they read q and k twice; 41 us more in them against 23 us for this kernel at 2048 rows x 8 heads of 128)
         const int n = b.v_off + a.heads * a.vdim - b.q_off;
-        k_silu_cols<<<(unsigned)(((size_t)R * n + 255) / 256), 256, 0, st>>>(m->P, l.n1, b.q_off, n, R);
+        pdl_launch(k_silu_cols, (unsigned)(((size_t)R * n + 255) / 256), 256, 0, st, m->P, l.n1, b.q_off, n, R);
         GTB_LAUNCHED();
     }
     auto post = [&]() -> int {
-        if (b.d.out_norm == 2) k_ret_post_all<OT><<<R, 256, 0, st>>>(a, b.d_onorm, m->O, m->P, l.n1, opC, l.kout_p);
-        else k_ret_post<OT><<<dim3(R, (a.heads + 3) / 4), 128, 0, st>>>(a, m->O, m->P, l.n1, opC, l.kout_p);
+        if (b.d.out_norm == 2) pdl_launch(k_ret_post_all<OT>, R, 256, 0, st, a, b.d_onorm, m->O, m->P, l.n1, opC, l.kout_p);
+        else pdl_launch(k_ret_post<OT>, dim3(R, (a.heads + 3) / 4), 128, 0, st, a, m->O, m->P, l.n1, opC, l.kout_p);
         GTB_LAUNCHED();
         return GTB_OK;
     };
@@ -605,7 +605,7 @@ int run_retention(gtb_seq_model* m, const PassTables& t, int R, int S, const Run
         if (need > m->retU_floats) return gtb::fail(GTB_ERR_STATE, "chunk workspace too small (%zu > %zu floats)", need, m->retU_floats);
         const int nvs = (a.vdim + rcfg.vs - 1) / rcfg.vs;
         if (a.rot_dims > 0 || a.scale != 1.0f) {
-            k_ret_rotate<<<R, 128, 0, st>>>(t, a, m->P, l.n1);
+            pdl_launch(k_ret_rotate, R, 128, 0, st, t, a, m->P, l.n1);
             GTB_LAUNCHED();
         }
         // wide value heads on aligned columns take the kernels with larger register tiles
@@ -615,28 +615,28 @@ int run_retention(gtb_seq_model* m, const PassTables& t, int R, int S, const Run
         if (wide) {
             constexpr size_t smem = 2 * RT_C * 128 * sizeof(float);
             GTB_CUDA(cudaFuncSetAttribute(k_ret_kv_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k_ret_kv_wide<<<wgrid, 256, smem, st>>>(t, a, m->P, l.n1, S, m->retU);
+            pdl_launch(k_ret_kv_wide, wgrid, 256, smem, st, t, a, m->P, l.n1, S, m->retU);
         } else {
             if (rcfg.smem_kv > 48 * 1024) GTB_CUDA(cudaFuncSetAttribute(k_ret_chunk_kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rcfg.smem_kv));
-            k_ret_chunk_kv<<<dim3(n_chunks, a.heads, nvs), 256, rcfg.smem_kv, st>>>(t, a, m->P, l.n1, S, rcfg.C, rcfg.vs, m->retU);
+            pdl_launch(k_ret_chunk_kv, dim3(n_chunks, a.heads, nvs), 256, rcfg.smem_kv, st, t, a, m->P, l.n1, S, rcfg.C, rcfg.vs, m->retU);
         }
         GTB_LAUNCHED();
-        if (quads) k_ret_scan<4><<<dim3(S, a.heads, (a.dim * a.vdim / 4 + 255) / 256), 256, 0, st>>>(t, a, S, rcfg.C, m->retU, run.state[bi]);
-        else k_ret_scan<1><<<dim3(S, a.heads, (a.dim * a.vdim + 255) / 256), 256, 0, st>>>(t, a, S, rcfg.C, m->retU, run.state[bi]);
+        if (quads) pdl_launch(k_ret_scan<4>, dim3(S, a.heads, (a.dim * a.vdim / 4 + 255) / 256), 256, 0, st, t, a, S, rcfg.C, m->retU, run.state[bi]);
+        else pdl_launch(k_ret_scan<1>, dim3(S, a.heads, (a.dim * a.vdim + 255) / 256), 256, 0, st, t, a, S, rcfg.C, m->retU, run.state[bi]);
         GTB_LAUNCHED();
         if (wide) {
             GTB_CUDA(cudaFuncSetAttribute(k_ret_out_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RT_OUT_SMEM));
-            k_ret_out_wide<<<wgrid, 256, RT_OUT_SMEM, st>>>(t, a, m->P, l.n1, S, m->retU, m->O);
+            pdl_launch(k_ret_out_wide, wgrid, 256, RT_OUT_SMEM, st, t, a, m->P, l.n1, S, m->retU, m->O);
         } else {
             if (rcfg.smem_out > 48 * 1024) GTB_CUDA(cudaFuncSetAttribute(k_ret_chunk_out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rcfg.smem_out));
-            k_ret_chunk_out<<<dim3(n_chunks, a.heads, nvs), 256, rcfg.smem_out, st>>>(t, a, m->P, l.n1, S, rcfg.C, rcfg.vs, m->retU, m->O);
+            pdl_launch(k_ret_chunk_out, dim3(n_chunks, a.heads, nvs), 256, rcfg.smem_out, st, t, a, m->P, l.n1, S, rcfg.C, rcfg.vs, m->retU, m->O);
         }
         GTB_LAUNCHED();
         return post();
     }
     const RetLaunch rl = ret_launch(b.d);
     if (rl.smem > 48 * 1024) GTB_CUDA(cudaFuncSetAttribute(k_retention, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rl.smem));
-    k_retention<<<dim3(S, a.heads, rl.nvs), rl.block, rl.smem, st>>>(t, a, m->P, l.n1, run.state[bi], m->O, rl.vs);
+    pdl_launch(k_retention, dim3(S, a.heads, rl.nvs), rl.block, rl.smem, st, t, a, m->P, l.n1, run.state[bi], m->O, rl.vs);
     GTB_LAUNCHED();
     return post();
 }
@@ -654,14 +654,14 @@ void sandwich_add(int R, size_t smem, const float* Y, const float* Y2, const flo
                   OT* op, int ld_op, const GroupRouteNext& rn, const JoinArgs* jn = nullptr) {
     cudaStream_t st = ctx().stream;
     if (jn) {
-        if (W <= 1024) k_sandwich_add<OT, 1, true><<<R, 256, smem, st>>>(Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, *jn);
-        else if (W <= 2048) k_sandwich_add<OT, 2, true><<<R, 256, smem, st>>>(Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, *jn);
-        else k_sandwich_add<OT, 4, true><<<R, 256, smem, st>>>(Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, *jn);
+        if (W <= 1024) pdl_launch(k_sandwich_add<OT, 1, true>, R, 256, smem, st, Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, *jn);
+        else if (W <= 2048) pdl_launch(k_sandwich_add<OT, 2, true>, R, 256, smem, st, Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, *jn);
+        else pdl_launch(k_sandwich_add<OT, 4, true>, R, 256, smem, st, Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, *jn);
         return;
     }
-    if (W <= 1024) k_sandwich_add<OT, 1><<<R, 256, smem, st>>>(Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, JoinArgs{});
-    else if (W <= 2048) k_sandwich_add<OT, 2><<<R, 256, smem, st>>>(Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, JoinArgs{});
-    else k_sandwich_add<OT, 4><<<R, 256, smem, st>>>(Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, JoinArgs{});
+    if (W <= 1024) pdl_launch(k_sandwich_add<OT, 1>, R, 256, smem, st, Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, JoinArgs{});
+    else if (W <= 2048) pdl_launch(k_sandwich_add<OT, 2>, R, 256, smem, st, Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, JoinArgs{});
+    else pdl_launch(k_sandwich_add<OT, 4>, R, 256, smem, st, Y, Y2, Yg, pair_dst, top, W, post, x, next, op, ld_op, rn, JoinArgs{});
 }
 
 // The convolution behind the q and k projections of a softmax-attention branch: convolved queries to m->convQ, keys (and plain values) to the
@@ -671,11 +671,11 @@ void launch_qk_conv(const PassTables& t, const ConvArgs& a, const float* P, int 
     const dim3 grid((R + rows_per - 1) / rows_per, ((a.nq + a.nk + a.nv) / V + 127) / 128);
     cudaStream_t st = ctx().stream;
     switch (a.taps) {
-        case 1: k_qk_conv<OT, V, 1><<<grid, 128, 0, st>>>(t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
-        case 2: k_qk_conv<OT, V, 2><<<grid, 128, 0, st>>>(t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
-        case 3: k_qk_conv<OT, V, 3><<<grid, 128, 0, st>>>(t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
-        case 4: k_qk_conv<OT, V, 4><<<grid, 128, 0, st>>>(t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
-        default: k_qk_conv<OT, V, 0><<<grid, 128, 0, st>>>(t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
+        case 1: pdl_launch(k_qk_conv<OT, V, 1>, grid, 128, 0, st, t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
+        case 2: pdl_launch(k_qk_conv<OT, V, 2>, grid, 128, 0, st, t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
+        case 3: pdl_launch(k_qk_conv<OT, V, 3>, grid, 128, 0, st, t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
+        case 4: pdl_launch(k_qk_conv<OT, V, 4>, grid, 128, 0, st, t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
+        default: pdl_launch(k_qk_conv<OT, V, 0>, grid, 128, 0, st, t, a, P, ldp, R, rows_per, tail, Q, kc, vc, every_one); break;
     }
 }
 template <typename OT>
@@ -692,7 +692,7 @@ int run_qk_conv(gtb_seq_model* m, const PassTables& t, int R, int S, const Run& 
     GTB_LAUNCHED();
     if (a.taps > 1 && !every_one) {
         const int nc = a.nq + a.nk;
-        k_canon_tail<<<dim3(S, (nc + 255) / 256), 256, 0, ctx().stream>>>(t, m->P + a.off, l.n1, nc, a.taps, run.ctail);
+        pdl_launch(k_canon_tail, dim3(S, (nc + 255) / 256), 256, 0, ctx().stream, t, m->P + a.off, l.n1, nc, a.taps, run.ctail);
         GTB_LAUNCHED();
     }
     return GTB_OK;
@@ -710,7 +710,7 @@ int run_soft_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const R
     const float* Q = m->P;                   // where the attention kernels read the queries
     int ldq = l.n1;
     if (a.qk_norm == 3) {
-        k_proj_rms<<<R, 256, 0, st>>>(m->P, l.n1, a.q_off, units * a.dim, a.k_off, nk * a.dim, c.eps, m->qk_sc);
+        pdl_launch(k_proj_rms, R, 256, 0, st, m->P, l.n1, a.q_off, units * a.dim, a.k_off, nk * a.dim, c.eps, m->qk_sc);
         GTB_LAUNCHED();
     }
     if (b.d.conv > 0) {
@@ -719,7 +719,7 @@ int run_soft_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const R
         Q = m->convQ; ldq = b.kq;
         a.q_off = 0; a.gate_src = m->P; a.gate_ld = l.n1;
     } else {
-        k_sattn_prep<OT><<<dim3(R, (units + nk + nv + 3) / 4), 128, 0, st>>>(t, a, m->P, l.n1, (OT*)run.kc[bi], (OT*)run.vc[bi]);
+        pdl_launch(k_sattn_prep<OT>, dim3(R, (units + nk + nv + 3) / 4), 128, 0, st, t, a, m->P, l.n1, (OT*)run.kc[bi], (OT*)run.vc[bi]);
         GTB_LAUNCHED();
     }
     // two maps per head: the units' outputs stay fp32 (their difference is taken afterwards), unit-major in m->O
@@ -739,17 +739,17 @@ int run_soft_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const R
         max_keys = std::min(c.max_ctx, max_keys + a.keep);
         const int splits = std::max(1, std::min(32, (max_keys + 127) / 128));
         if (splits > 1) {
-            k_sattn_split<OT><<<dim3(R, units, splits), 128, smem, st>>>(t, a, Q, ldq, (const OT*)run.kc[bi], (const OT*)run.vc[bi], nullptr, nullptr, m->sattn_part, R);
+            pdl_launch(k_sattn_split<OT>, dim3(R, units, splits), 128, smem, st, t, a, Q, ldq, (const OT*)run.kc[bi], (const OT*)run.vc[bi], nullptr, nullptr, m->sattn_part, R);
             GTB_LAUNCHED();
-            if (of) k_sattn_join<float><<<dim3(R, units), 128, 0, st>>>(af, Q, ldq, m->sattn_part, R, splits, of, ldf);
-            else k_sattn_join<OT><<<dim3(R, units), 128, 0, st>>>(a, Q, ldq, m->sattn_part, R, splits, opC, l.kout_p);
+            if (of) pdl_launch(k_sattn_join<float>, dim3(R, units), 128, 0, st, af, Q, ldq, m->sattn_part, R, splits, of, ldf);
+            else pdl_launch(k_sattn_join<OT>, dim3(R, units), 128, 0, st, a, Q, ldq, m->sattn_part, R, splits, opC, l.kout_p);
             GTB_LAUNCHED();
             done = 0;
         }
     }
     if (done < 0) {
-        if (of) k_sattn<OT, float><<<dim3(R, units), 128, smem, st>>>(t, af, Q, ldq, (const OT*)run.kc[bi], (const OT*)run.vc[bi], nullptr, nullptr, of, ldf);
-        else k_sattn<OT, OT><<<dim3(R, units), 128, smem, st>>>(t, a, Q, ldq, (const OT*)run.kc[bi], (const OT*)run.vc[bi], nullptr, nullptr, opC, l.kout_p);
+        if (of) pdl_launch(k_sattn<OT, float>, dim3(R, units), 128, smem, st, t, af, Q, ldq, (const OT*)run.kc[bi], (const OT*)run.vc[bi], nullptr, nullptr, of, ldf);
+        else pdl_launch(k_sattn<OT, OT>, dim3(R, units), 128, smem, st, t, a, Q, ldq, (const OT*)run.kc[bi], (const OT*)run.vc[bi], nullptr, nullptr, opC, l.kout_p);
         GTB_LAUNCHED();
     }
     if (of) {
@@ -757,7 +757,7 @@ int run_soft_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const R
         d.heads = a.heads; d.dim = a.dim; d.vdim = a.vdim; d.diff = b.d.diff; d.eps = c.eps; d.out_scale = b.d.out_scale != 0.0f ? b.d.out_scale : 1.0f;
         d.lq1 = b.d_lam[0]; d.lk1 = b.d_lam[1]; d.lq2 = b.d_lam[2]; d.lk2 = b.d_lam[3];
         d.gate = b.d.gated; d.g_off = b.g_off; d.a_off = b.a_off;
-        k_diff_combine<OT><<<dim3(R, (a.heads + 3) / 4), 128, 0, st>>>(d, of, m->P, l.n1, opC, l.kout_p);
+        pdl_launch(k_diff_combine<OT>, dim3(R, (a.heads + 3) / 4), 128, 0, st, d, of, m->P, l.n1, opC, l.kout_p);
         GTB_LAUNCHED();
     }
     return GTB_OK;
@@ -775,7 +775,7 @@ int run_act_conv(gtb_seq_model* m, const PassTables& t, int R, int S, const Run&
     else launch_qk_conv<OT, 1>(t, a, m->P, l.n1, R, rows_per, run.ctail, m->convQ, (OT*)nullptr, (OT*)nullptr, every_one);
     GTB_LAUNCHED();
     if (a.taps > 1 && !every_one) {
-        k_canon_tail<<<dim3(S, (nq + 255) / 256), 256, 0, ctx().stream>>>(t, m->P + off, l.n1, nq, a.taps, run.ctail);
+        pdl_launch(k_canon_tail, dim3(S, (nq + 255) / 256), 256, 0, ctx().stream, t, m->P + off, l.n1, nq, a.taps, run.ctail);
         GTB_LAUNCHED();
     }
     return GTB_OK;
@@ -794,8 +794,8 @@ RecBranch rec_args(const gtb_seq_model* m, const BranchW& b) {
 template <int KIND, int RPT>
 void launch_rec_walk_n(const PassTables& t, const RecBranch& a, int S, bool one, const float* X, int ldx, const float* P, int ldp, const float4* G, const float* ms, float* state, float* O) {
     const dim3 grid(S, a.heads, (a.vx + 31) / 32);
-    if (one) k_rec_walk<KIND, RPT, true><<<grid, 256, 0, ctx().stream>>>(t, a, X, ldx, P, ldp, G, ms, state, O);
-    else k_rec_walk<KIND, RPT, false><<<grid, 256, 0, ctx().stream>>>(t, a, X, ldx, P, ldp, G, ms, state, O);
+    if (one) pdl_launch(k_rec_walk<KIND, RPT, true>, grid, 256, 0, ctx().stream, t, a, X, ldx, P, ldp, G, ms, state, O);
+    else pdl_launch(k_rec_walk<KIND, RPT, false>, grid, 256, 0, ctx().stream, t, a, X, ldx, P, ldp, G, ms, state, O);
 }
 template <int KIND>
 int launch_rec_walk(const PassTables& t, const RecBranch& a, int S, bool one, const float* X, int ldx, const float* P, int ldp, const float4* G, const float* ms, float* state, float* O) {
@@ -813,7 +813,7 @@ int launch_rec_scan(gtb_seq_model* m, const PassTables& t, const RecBranch& a, i
     const size_t smem = ((size_t)(KIND == REC_DELTA ? 8 : 4) * C * (a.dp + 8) + 2 * (size_t)a.dp * (REC_VS + 8) + 2 * C * (REC_VS + 8)) * 2;
     static size_t allowed = 40 * 1024;      // (beside static shared memory)
     if (smem > allowed) { GTB_CUDA(cudaFuncSetAttribute(k_rec_scan<KIND, C, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); allowed = smem; }
-    k_rec_scan<KIND, C, MT><<<dim3(S, a.heads, a.vp / REC_VS), 256, smem, ctx().stream>>>(t, a, m->recK, ps_qk, m->recW, ps_w, m->recG, m->recB, X, ldx, m->recV, ps_v, m->recS, state);
+    pdl_launch(k_rec_scan<KIND, C, MT>, dim3(S, a.heads, a.vp / REC_VS), 256, smem, ctx().stream, t, a, m->recK, ps_qk, m->recW, ps_w, m->recG, m->recB, X, ldx, m->recV, ps_v, m->recS, state);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -822,7 +822,7 @@ int launch_rec_out(gtb_seq_model* m, const PassTables& t, const RecBranch& a, in
     const size_t smem = (4 * (size_t)C * 72 + 2 * 64 * (size_t)(VP + 8)) * 2;
     static bool attr = false;
     if (!attr) { GTB_CUDA(cudaFuncSetAttribute(k_rec_out<VP, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr = true; }
-    k_rec_out<VP, C><<<dim3(n_chunks, a.heads, (a.vp + VP - 1) / VP), 2 * C, smem, ctx().stream>>>(t, a, kind, S, m->recQ, m->recK, ps_qk, m->recV, ps_v, m->recS, m->recG, m->recB, m->O);
+    pdl_launch(k_rec_out<VP, C>, dim3(n_chunks, a.heads, (a.vp + VP - 1) / VP), 2 * C, smem, ctx().stream, t, a, kind, S, m->recQ, m->recK, ps_qk, m->recV, ps_v, m->recS, m->recG, m->recB, m->O);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -831,13 +831,13 @@ int run_rec_chunks(gtb_seq_model* m, const PassTables& t, const RecBranch& a, in
     cudaStream_t st = ctx().stream;
     const size_t ps_qk = (size_t)m->max_rows * a.kv_heads * a.dp, ps_w = (size_t)m->max_rows * a.heads * a.dp, ps_v = (size_t)m->max_rows * a.heads * a.vp;
     const int units = 2 * a.kv_heads + a.heads;
-    k_rec_prep<KIND><<<dim3(R, (units + 7) / 8), 256, 0, st>>>(a, X, ldx, m->recQ, m->recK, ps_qk, m->recV, ps_v);
+    pdl_launch(k_rec_prep<KIND>, dim3(R, (units + 7) / 8), 256, 0, st, a, X, ldx, m->recQ, m->recK, ps_qk, m->recV, ps_v);
     GTB_LAUNCHED();
     if (KIND == REC_DELTA) {
         const size_t smem = 2 * (size_t)C * (C + 4) * sizeof(float) + 2 * (size_t)C * (std::max(a.dp, a.vp) + 8) * 2;
         static size_t allowed = 40 * 1024;      // (beside static shared memory)
         if (smem > allowed) { GTB_CUDA(cudaFuncSetAttribute(k_delta_wy<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); allowed = smem; }
-        k_delta_wy<C><<<dim3(n_chunks, a.heads), 256, smem, st>>>(t, a, S, m->recK, ps_qk, m->recV, ps_v, m->recG, m->recB, X, ldx, m->recW, ps_w);
+        pdl_launch(k_delta_wy<C>, dim3(n_chunks, a.heads), 256, smem, st, t, a, S, m->recK, ps_qk, m->recV, ps_v, m->recG, m->recB, X, ldx, m->recW, ps_w);
         GTB_LAUNCHED();
     }
     int rc = a.dp <= 128 ? launch_rec_scan<KIND, C, 1>(m, t, a, S, ps_qk, ps_w, ps_v, X, ldx, state) : launch_rec_scan<KIND, C, 2>(m, t, a, S, ps_qk, ps_w, ps_v, X, ldx, state);
@@ -866,7 +866,7 @@ int run_rec_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const Ru
     const bool chunks = sizeof(OT) == 2 && portions && C > 0;
     const bool one = R == S;                     // every segment is one row: gates and unit lengths inside the walk
     if (!one) {
-        k_rec_gates<KIND><<<dim3(S, a.heads), R >= 512 * S ? 1024 : chunks || R >= 64 * S ? 256 : 64, 0, st>>>(t, a, m->P, l.n1, C, run.mstate[bi], m->recG, chunks ? m->recB : nullptr);
+        pdl_launch(k_rec_gates<KIND>, dim3(S, a.heads), R >= 512 * S ? 1024 : chunks || R >= 64 * S ? 256 : 64, 0, st, t, a, m->P, l.n1, C, run.mstate[bi], m->recG, chunks ? m->recB : nullptr);
         GTB_LAUNCHED();
     }
     int rc;
@@ -877,13 +877,13 @@ int run_rec_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const Ru
         rc = C == 64 ? run_rec_chunks<KIND, 64>(m, t, a, R, S, n_chunks, X, ldx, run.state[bi]) : run_rec_chunks<KIND, 32>(m, t, a, R, S, n_chunks, X, ldx, run.state[bi]);
     } else {
         if (KIND == REC_DELTA && !one) {
-            k_rec_unit<<<dim3(R, (2 * a.kv_heads + 3) / 4), 128, 0, st>>>(a, X, ldx);
+            pdl_launch(k_rec_unit, dim3(R, (2 * a.kv_heads + 3) / 4), 128, 0, st, a, X, ldx);
             GTB_LAUNCHED();
         }
         rc = launch_rec_walk<KIND>(t, a, S, one, X, ldx, m->P, l.n1, m->recG, run.mstate[bi], run.state[bi], m->O);
     }
     if (rc) return rc;
-    k_rec_post<OT, KIND><<<dim3(R, (a.heads + 3) / 4), 128, 0, st>>>(t, a, m->O, one ? nullptr : m->recG, run.mstate[bi], m->P, l.n1, (OT*)m->opC, l.kout_p);
+    pdl_launch(k_rec_post<OT, KIND>, dim3(R, (a.heads + 3) / 4), 128, 0, st, t, a, m->O, one ? nullptr : m->recG, run.mstate[bi], m->P, l.n1, (OT*)m->opC, l.kout_p);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -891,7 +891,7 @@ int run_rec_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const Ru
 template <typename OT, int LANES, int KS, int TILE>
 int launch_ssm(const PassTables& t, const SsmBranch& a, int S, const float* XC, const float* DT, const float* BC, int ld_bc, const float* P, int ldp, float* state, OT* out, int ld_out) {
     constexpr int NCH = 128 / LANES;
-    k_ssm_scan<OT, LANES, KS, TILE><<<dim3(S, (a.inner + NCH - 1) / NCH), 128 + SSM_SERVE, 0, ctx().stream>>>(t, a, XC, DT, BC, ld_bc, P, ldp, state, out, ld_out);
+    pdl_launch(k_ssm_scan<OT, LANES, KS, TILE>, dim3(S, (a.inner + NCH - 1) / NCH), 128 + SSM_SERVE, 0, ctx().stream, t, a, XC, DT, BC, ld_bc, P, ldp, state, out, ld_out);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -908,7 +908,7 @@ int run_ssm_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const Ru
     rc = product<OT>(m, m->opX, b.ld_x, b.w_x, b.ld_x, m->ssmBC, b.ld_bc, R, nbc, b.ld_x, nullptr, 0);
     if (rc) return rc;
     if (sizeof(OT) == 2 && m->use_tensor && m->gp && R >= m->tensor_min_rows) {
-        k_cols_operand<OT><<<R, 64, 0, st>>>(m->ssmBC, b.ld_bc, a.dt_rank, (OT*)m->opDT, b.dt_p);
+        pdl_launch(k_cols_operand<OT>, R, 64, 0, st, m->ssmBC, b.ld_bc, a.dt_rank, (OT*)m->opDT, b.dt_p);
         GTB_LAUNCHED();
         rc = product<OT>(m, m->opDT, b.dt_p, b.w_dt, b.dt_p, m->ssmDT, a.inner, R, a.inner, b.dt_p, b.d_dtb, 0);
     } else rc = product<float>(m, m->ssmBC, b.ld_bc, b.w_dt, b.dt_p, m->ssmDT, a.inner, R, a.inner, b.dt_p, b.d_dtb, 0);    // (the columns behind dt_rank meet zero weights)
@@ -945,7 +945,7 @@ int launch_lat_dec_mma(const PassTables& t, const SoftAttn& a, int R, int splits
     static size_t allowed = 48 * 1024;
     if (smem > 200 * 1024) return -1;
     if (smem > allowed) { GTB_CUDA(cudaFuncSetAttribute(k_lat_dec_mma<VPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); allowed = smem; }
-    k_lat_dec_mma<VPW><<<dim3(R, (a.heads + 15) / 16, splits), 128, smem, ctx().stream>>>(t, a, QA, ldqa, cache, part, R);
+    pdl_launch(k_lat_dec_mma<VPW>, dim3(R, (a.heads + 15) / 16, splits), 128, smem, ctx().stream, t, a, QA, ldqa, cache, part, R);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -972,7 +972,7 @@ int run_latent_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const
     const int hd = a.dim + a.rope, parts = (a.own_kv ? 1 : 0) + (a.q_rank > 0 ? 1 : 0);
     int rc;
     if (parts > 0) {
-        k_lat_prep<OT><<<dim3(R, parts), 128, 0, st>>>(t, a, m->P, l.n1, (OT*)run.kc[0], (OT*)m->opQ, b.qrank_p);
+        pdl_launch(k_lat_prep<OT>, dim3(R, parts), 128, 0, st, t, a, m->P, l.n1, (OT*)run.kc[0], (OT*)m->opQ, b.qrank_p);
         GTB_LAUNCHED();
     }
     const float* Q = m->P;
@@ -985,7 +985,7 @@ int run_latent_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const
     }
     if (expand) {
         const int ld_qr = a.heads * hd, nx = a.heads * (a.dim + a.vdim);
-        k_lat_qrot<<<R, 128, 0, st>>>(t, a, Q, ldq, q0, m->latQ, ld_qr);
+        pdl_launch(k_lat_qrot, R, 128, 0, st, t, a, Q, ldq, q0, m->latQ, ld_qr);
         GTB_LAUNCHED();
         for (int s = 0; s < S; s++) {
             const int slot = seg_slots[s], p0 = m->host_pos[slot];
@@ -993,7 +993,7 @@ int run_latent_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const
             const bf16* src = (const bf16*)run.kc[0] + ((size_t)slot * c.max_ctx + lo) * b.c_ld;
             rc = product<OT>(m, src, b.c_ld, b.w_uk, b.rank_p, m->latX, nx, n, nx, b.rank_p, nullptr, 0);      // uk and uv rows are one matrix
             if (rc) return rc;
-            k_lat_pack<<<n, 256, 0, st>>>(a, m->latX, n, slot, lo, (const bf16*)run.kc[0], m->latKx, m->latVx);
+            pdl_launch(k_lat_pack, n, 256, 0, st, a, m->latX, n, slot, lo, (const bf16*)run.kc[0], m->latKx, m->latVx);
             GTB_LAUNCHED();
         }
         SoftAttn sa{};
@@ -1003,7 +1003,7 @@ int run_latent_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const
         if (rc < 0) return gtb::fail(GTB_ERR_STATE, "head sizes outside the tiled attention kernel");
         return rc;
     }
-    k_lat_qabs<<<dim3(R, a.heads, (a.rank + 127) / 128), 128, (hd + 512) * sizeof(float), st>>>(t, a, Q, ldq, q0, b.w_uk, b.rank_p, m->latQA);
+    pdl_launch(k_lat_qabs, dim3(R, a.heads, (a.rank + 127) / 128), 128, (hd + 512) * sizeof(float), st, t, a, Q, ldq, q0, b.w_uk, b.rank_p, m->latQA);
     GTB_LAUNCHED();
     const SoftAttn sa = lat_soft_args(m, b);
     const int ldqa = a.heads * sa.dim, ld_ol = (a.heads * a.rank + 7) / 8 * 8;
@@ -1016,7 +1016,7 @@ int run_latent_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const
         rc = lat_dec_mma(t, sa, R, splits, m->latQA, ldqa, (const bf16*)run.kc[0], m->sattn_part);
         if (rc > 0) return rc;
         if (rc == 0) {
-            k_sattn_join<OT><<<dim3(R, sa.heads), 128, 0, st>>>(sa, m->latQA, ldqa, m->sattn_part, R, splits, (OT*)m->opO, ld_ol);
+            pdl_launch(k_sattn_join<OT>, dim3(R, sa.heads), 128, 0, st, sa, m->latQA, ldqa, m->sattn_part, R, splits, (OT*)m->opO, ld_ol);
             GTB_LAUNCHED();
             done = true;
         }
@@ -1025,19 +1025,19 @@ int run_latent_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const
         const int max_keys = sa.window > 0 ? std::min(c.max_ctx, sa.window) : c.max_ctx;
         const int splits = std::max(1, std::min(32, (max_keys + 127) / 128));
         if (splits > 1) {
-            k_sattn_split<OT><<<dim3(R, sa.heads, splits), 128, smem, st>>>(t, sa, m->latQA, ldqa, (const OT*)run.kc[0], (const OT*)run.kc[0], nullptr, nullptr, m->sattn_part, R);
+            pdl_launch(k_sattn_split<OT>, dim3(R, sa.heads, splits), 128, smem, st, t, sa, m->latQA, ldqa, (const OT*)run.kc[0], (const OT*)run.kc[0], nullptr, nullptr, m->sattn_part, R);
             GTB_LAUNCHED();
-            k_sattn_join<OT><<<dim3(R, sa.heads), 128, 0, st>>>(sa, m->latQA, ldqa, m->sattn_part, R, splits, (OT*)m->opO, ld_ol);
+            pdl_launch(k_sattn_join<OT>, dim3(R, sa.heads), 128, 0, st, sa, m->latQA, ldqa, m->sattn_part, R, splits, (OT*)m->opO, ld_ol);
             GTB_LAUNCHED();
             done = true;
         }
     }
     if (!done) {
-        k_sattn<OT><<<dim3(R, sa.heads), 128, smem, st>>>(t, sa, m->latQA, ldqa, (const OT*)run.kc[0], (const OT*)run.kc[0], nullptr, nullptr, (OT*)m->opO, ld_ol);
+        pdl_launch(k_sattn<OT>, dim3(R, sa.heads), 128, smem, st, t, sa, m->latQA, ldqa, (const OT*)run.kc[0], (const OT*)run.kc[0], nullptr, nullptr, (OT*)m->opO, ld_ol);
         GTB_LAUNCHED();
     }
     const int n_out = a.heads * a.vdim;
-    k_lat_vup<OT><<<dim3(R, std::max(1, std::min(std::max(1, 4096 / R), (n_out + 7) / 8))), 256, 0, st>>>(a, (const OT*)m->opO, ld_ol, b.w_uv, b.rank_p, m->P, l.n1, b.d.gated, opC, l.kout_p);
+    pdl_launch(k_lat_vup<OT>, dim3(R, std::max(1, std::min(std::max(1, 4096 / R), (n_out + 7) / 8))), 256, 0, st, a, (const OT*)m->opO, ld_ol, b.w_uv, b.rank_p, m->P, l.n1, b.d.gated, opC, l.kout_p);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -1058,8 +1058,8 @@ int run_gated_experts(gtb_seq_model* m, int R, const LayerW& l, bool is_routed, 
     if (!is_routed) {                        // router (and the shared expert's gate) in one product, fp32 accumulation
         rc = product<OT>(m, opA, wp, l.w_router, wp, m->rl, l.n_out, R, l.n_out, wp, nullptr, 0);
         if (rc) return rc;
-        if (l.d.route_kind == GTB_ROUTE_SOFTMAX) k_moe_route_softmax<<<R, 32, E * sizeof(float), st>>>(m->rl, l.n_out, E, top, m->sel_idx, m->sel_w);
-        else k_moe_route_sigmoid<<<R, 32, E * sizeof(float), st>>>(m->rl, l.n_out, E, top, m->sel_idx, m->sel_w, l.sff > 0 ? m->shw : nullptr);
+        if (l.d.route_kind == GTB_ROUTE_SOFTMAX) pdl_launch(k_moe_route_softmax, R, 32, E * sizeof(float), st, m->rl, l.n_out, E, top, m->sel_idx, m->sel_w);
+        else pdl_launch(k_moe_route_sigmoid, R, 32, E * sizeof(float), st, m->rl, l.n_out, E, top, m->sel_idx, m->sel_w, l.sff > 0 ? m->shw : nullptr);
         GTB_LAUNCHED();
     }
     if (l.sff > 0) {
@@ -1072,7 +1072,7 @@ int run_gated_experts(gtb_seq_model* m, int R, const LayerW& l, bool is_routed, 
         if (!act_done) {
             rc = product<OT>(m, opA, wp, l.w_sh_gu, wp, m->G, 2 * l.sff, R, 2 * l.sff, wp, nullptr, 0);
             if (rc) return rc;
-            k_swiglu_rows<OT><<<dim3(R, std::max(1, std::min((l.sff_p + 255) / 256, std::max(1, 2048 / R)))), 256, 0, st>>>(m->G, l.sff, l.sh_inter ? 1 : 0, m->shw, opC, l.sff_p);
+            pdl_launch(k_swiglu_rows<OT>, dim3(R, std::max(1, std::min((l.sff_p + 255) / 256, std::max(1, 2048 / R)))), 256, 0, st, m->G, l.sff, l.sh_inter ? 1 : 0, m->shw, opC, l.sff_p);
             GTB_LAUNCHED();
         }
         rc = product<OT>(m, opC, l.sff_p, l.w_sh_down, l.sff_p, m->Y2, W, R, W, l.sff_p, nullptr, 0);
@@ -1083,9 +1083,9 @@ int run_gated_experts(gtb_seq_model* m, int R, const LayerW& l, bool is_routed, 
     if (sizeof(OT) == 2 && m->grouped_experts && m->use_tensor && m->gp && m->Xg && l.e_inter && R >= m->tensor_min_rows && mpad <= m->mpad_max) {
         // rows sorted by expert; the gate-and-up product writes w * silu(gate) * up per (row, choice), the down product one output row per pair,
         // and the residual update sums a row's pairs
-        k_moe_group<<<1, 1024, 2 * E * sizeof(int), st>>>(m->sel_idx, n_pairs, E, m->pair_dst, m->tile_e, mpad / 128);
+        pdl_launch(k_moe_group, 1, 1024, 2 * E * sizeof(int), st, m->sel_idx, n_pairs, E, m->pair_dst, m->tile_e, mpad / 128);
         GTB_LAUNCHED();
-        k_moe_gather<<<n_pairs, 128, 0, st>>>((const bf16*)opA, wp, top, m->pair_dst, m->sel_w, m->Xg, m->rw);
+        pdl_launch(k_moe_gather, n_pairs, 128, 0, st, (const bf16*)opA, wp, top, m->pair_dst, m->sel_w, m->Xg, m->rw);
         GTB_LAUNCHED();
         rc = seq_gemm_bf16_grouped_gated(m->gp, m->Xg, wp, l.w_up, wp, mpad, 2 * l.ff, wp, E, m->tile_e, m->actg, l.kfp, m->rw, 1);
         if (rc == 0) rc = seq_gemm_bf16_grouped(m->gp, m->actg, l.kfp, l.w_down, l.kfp, mpad, W, l.kfp, E, m->tile_e, m->Yg, W, nullptr, 0, nullptr);
@@ -1096,9 +1096,9 @@ int run_gated_experts(gtb_seq_model* m, int R, const LayerW& l, bool is_routed, 
         }
     }
     const int cta_budget = std::max(1, 4096 / std::max(1, R * top));
-    k_moe_gu_rows<OT><<<dim3(R * top, std::max(1, std::min(cta_budget, (l.kfp + 7) / 8))), 256, 0, st>>>(opA, wp, wp, l.w_up, wp, l.ff, l.kfp, l.e_inter ? 1 : 0, top, m->sel_idx, m->sel_w, (OT*)m->act);
+    pdl_launch(k_moe_gu_rows<OT>, dim3(R * top, std::max(1, std::min(cta_budget, (l.kfp + 7) / 8))), 256, 0, st, opA, wp, wp, l.w_up, wp, l.ff, l.kfp, l.e_inter ? 1 : 0, top, m->sel_idx, m->sel_w, (OT*)m->act);
     GTB_LAUNCHED();
-    k_moe_down_rows<OT><<<dim3(R, std::max(1, std::min(std::max(1, 4096 / R), (W + 7) / 8))), 256, 0, st>>>((const OT*)m->act, l.kfp, l.w_down, W, E, top, m->sel_idx, m->Y, W);
+    pdl_launch(k_moe_down_rows<OT>, dim3(R, std::max(1, std::min(std::max(1, 4096 / R), (W + 7) / 8))), 256, 0, st, (const OT*)m->act, l.kfp, l.w_down, W, E, top, m->sel_idx, m->Y, W);
     GTB_LAUNCHED();
     eo.Y = m->Y;
     return GTB_OK;
@@ -1168,17 +1168,17 @@ int run_sandwich_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
         if (!act_done && R <= 8) {          // few rows: the activation leaves the weight-streaming product
             const OT* a = opA;
             const dim3 grid((l.ff + 3) / 4);
-            if (R <= 1) k_gemv_rows<OT, 1, 4, true, OT><<<grid, 256, 0, st>>>(a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
-            else if (R <= 2) k_gemv_rows<OT, 2, 4, true, OT><<<grid, 256, 0, st>>>(a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
-            else if (R <= 4) k_gemv_rows<OT, 4, 4, true, OT><<<grid, 256, 0, st>>>(a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
-            else k_gemv_rows<OT, 8, 4, true, OT><<<grid, 256, 0, st>>>(a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
+            if (R <= 1) pdl_launch(k_gemv_rows<OT, 1, 4, true, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
+            else if (R <= 2) pdl_launch(k_gemv_rows<OT, 2, 4, true, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
+            else if (R <= 4) pdl_launch(k_gemv_rows<OT, 4, 4, true, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
+            else pdl_launch(k_gemv_rows<OT, 8, 4, true, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
             GTB_LAUNCHED();
             act_done = true;
         }
         if (!act_done) {
             rc = product<OT>(m, opA, wp, l.w_up, wp, m->G, l.ff, R, l.ff, wp, nullptr, 0);
             if (rc) return rc;
-            k_gelu_rows<OT><<<dim3(R, std::max(1, std::min((l.kfp + 255) / 256, std::max(1, 2048 / R)))), 256, 0, st>>>(m->G, l.ff, opC, l.kfp);
+            pdl_launch(k_gelu_rows<OT>, dim3(R, std::max(1, std::min((l.kfp + 255) / 256, std::max(1, 2048 / R)))), 256, 0, st, m->G, l.ff, opC, l.kfp);
             GTB_LAUNCHED();
         }
         rc = product<OT>(m, opC, l.kfp, l.w_down, l.kfp, m->Y, W, R, W, l.kfp, nullptr, 0);
@@ -1197,7 +1197,7 @@ int run_sandwich_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
         if (!act_done) {
             rc = product<OT>(m, opA, wp, l.w_gu, wp, m->G, 2 * l.ff, R, 2 * l.ff, wp, nullptr, 0);
             if (rc) return rc;
-            k_swiglu_rows<OT><<<dim3(R, std::max(1, std::min((l.kfp + 255) / 256, std::max(1, 2048 / R)))), 256, 0, st>>>(m->G, l.ff, l.gu_inter ? 1 : 0, nullptr, opC, l.kfp);
+            pdl_launch(k_swiglu_rows<OT>, dim3(R, std::max(1, std::min((l.kfp + 255) / 256, std::max(1, 2048 / R)))), 256, 0, st, m->G, l.ff, l.gu_inter ? 1 : 0, nullptr, opC, l.kfp);
             GTB_LAUNCHED();
         }
         rc = product<OT>(m, opC, l.kfp, l.w_down, l.kfp, m->Y, W, R, W, l.kfp, nullptr, 0);
@@ -1211,14 +1211,14 @@ int run_sandwich_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
     if (!rn.w) {
         rc = product<OT>(m, opA, wp, l.w_router, wp, m->rl, E, R, E, wp, nullptr, 0);
         if (rc) return rc;
-        k_moe_route_grouped<<<R, 32, (2 * E + groups) * sizeof(float), st>>>(m->rl, E, E, groups, keep, l.d.top, l.d.route_scale, l.n_sh, m->sel_idx, m->sel_w);
+        pdl_launch(k_moe_route_grouped, R, 32, (2 * E + groups) * sizeof(float), st, m->rl, E, E, groups, keep, l.d.top, l.d.route_scale, l.n_sh, m->sel_idx, m->sel_w);
         GTB_LAUNCHED();
     }
     const int n_pairs = R * top, mpad = (n_pairs + 127) / 128 * 128 + Et * 128;
     if (sizeof(OT) == 2 && m->grouped_experts && m->use_tensor && m->gp && m->Xg && R >= m->tensor_min_rows && mpad <= m->mpad_max) {
-        k_moe_group<<<1, 1024, 2 * Et * sizeof(int), st>>>(m->sel_idx, n_pairs, Et, m->pair_dst, m->tile_e, mpad / 128);
+        pdl_launch(k_moe_group, 1, 1024, 2 * Et * sizeof(int), st, m->sel_idx, n_pairs, Et, m->pair_dst, m->tile_e, mpad / 128);
         GTB_LAUNCHED();
-        k_moe_gather<<<n_pairs, 128, 0, st>>>((const bf16*)opA, wp, top, m->pair_dst, m->sel_w, m->Xg, m->rw);
+        pdl_launch(k_moe_gather, n_pairs, 128, 0, st, (const bf16*)opA, wp, top, m->pair_dst, m->sel_w, m->Xg, m->rw);
         GTB_LAUNCHED();
         rc = seq_gemm_bf16_grouped(m->gp, m->Xg, wp, l.w_up, wp, mpad, l.ff, wp, Et, m->tile_e, nullptr, 0, m->actg, l.kfp, m->rw);
         if (rc == 0) rc = seq_gemm_bf16_grouped(m->gp, m->actg, l.kfp, l.w_down, l.kfp, mpad, W, l.kfp, Et, m->tile_e, m->Yg, W, nullptr, 0, nullptr);
@@ -1230,9 +1230,9 @@ int run_sandwich_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
         }
     }
     const int cta_budget = std::max(1, 4096 / std::max(1, R * top));
-    k_moe_up_rows<OT><<<dim3(R * top, std::max(1, std::min(cta_budget, (l.kfp + 7) / 8))), 256, 0, st>>>(opA, wp, wp, l.w_up, wp, l.ff, l.kfp, Et, top, m->sel_idx, m->sel_w, (OT*)m->act);
+    pdl_launch(k_moe_up_rows<OT>, dim3(R * top, std::max(1, std::min(cta_budget, (l.kfp + 7) / 8))), 256, 0, st, opA, wp, wp, l.w_up, wp, l.ff, l.kfp, Et, top, m->sel_idx, m->sel_w, (OT*)m->act);
     GTB_LAUNCHED();
-    k_moe_down_rows<OT><<<dim3(R, std::max(1, std::min(std::max(1, 4096 / R), (W + 7) / 8))), 256, 0, st>>>((const OT*)m->act, l.kfp, l.w_down, W, Et, top, m->sel_idx, m->Y, W);
+    pdl_launch(k_moe_down_rows<OT>, dim3(R, std::max(1, std::min(std::max(1, 4096 / R), (W + 7) / 8))), 256, 0, st, (const OT*)m->act, l.kfp, l.w_down, W, Et, top, m->sel_idx, m->Y, W);
     GTB_LAUNCHED();
     sandwich_add<OT>(R, 0, m->Y, nullptr, nullptr, nullptr, 0, W, sw_norm(m, l, 3), m->x, next, opA, wp, GroupRouteNext{});
     GTB_LAUNCHED();
@@ -1259,7 +1259,7 @@ int hc_boundary(gtb_seq_model* m, int R, PendingUpdate& pend, const float* hc_ne
     const bool whole_row = hc_next && nrm.kind == GTB_NORM_RMS;       // the RMS norm sums over the row inside one CTA
     const int V = W % 4 == 0 ? 4 : 1;
     const int gy = whole_row ? 1 : std::max(1, std::min((W / V + 255) / 256, std::max(1, 2048 / R)));
-#define HC_LAUNCH(VV, NN) k_hc_step<OT, VV, NN><<<dim3(R, gy), 256, 0, ctx().stream>>>(m->xs, (size_t)m->max_rows * W, m->ns, pend.src_ns, W, pend.Y, pend.Y2, pend.Yg, \
+#define HC_LAUNCH(VV, NN) pdl_launch(k_hc_step<OT, VV, NN>, dim3(R, gy), 256, 0, ctx().stream, m->xs, (size_t)m->max_rows * W, m->ns, pend.src_ns, W, pend.Y, pend.Y2, pend.Yg, \
                                                                                       pend.pair_dst, pend.top, pend.hc, hc_next, nrm, (OT*)m->opA, m->wp, xsum)
     if (V == 4) { if (m->ns <= 2) HC_LAUNCH(4, 2); else if (m->ns <= 4) HC_LAUNCH(4, 4); else HC_LAUNCH(4, 8); }
     else { if (m->ns <= 2) HC_LAUNCH(1, 2); else if (m->ns <= 4) HC_LAUNCH(1, 4); else HC_LAUNCH(1, 8); }
@@ -1302,7 +1302,7 @@ int run_prenorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, const
             rc = product<OT>(m, opA, wp, l.w_gu, wp, m->G, 2 * l.ff, R, 2 * l.ff, wp, nullptr, 0);
             if (rc) return rc;
             const size_t n = (size_t)R * l.ff;
-            k_geglu<OT><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(m->G, l.ff, opC, l.kfp, 0, R, l.gu_inter ? 1 : 0);
+            pdl_launch(k_geglu<OT>, (unsigned)((n + 255) / 256), 256, 0, st, m->G, l.ff, opC, l.kfp, 0, R, l.gu_inter ? 1 : 0);
             GTB_LAUNCHED();
         }
         rc = product<OT>(m, opC, l.kfp, l.w_down, l.kfp, m->Y, W, R, W, l.kfp, nullptr, 0);
@@ -1329,19 +1329,19 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
     const bool portions = seg_lens != nullptr && m->fused_attn && R >= 16 * S;
     int n_qtiles = 0;
     if (portions) for (int s = 0; s < S; s++) n_qtiles += (seg_lens[s] + 63) / 64;
-    k_plan<<<(R + 127) / 128, 128, 0, st>>>(t, R, from_pending ? 1 : 0);
+    pdl_launch(k_plan, (R + 127) / 128, 128, 0, st, t, R, from_pending ? 1 : 0);
     GTB_LAUNCHED();
     const bool first_reads_x = m->L[m->runs[0].layer].d.style == GTB_BLOCK_POSTNORM;
     const float emb_scale = c.embed_scale != 0.0f ? c.embed_scale : 1.0f;
     if (m->sandwich && c.bigram_buckets == 0) {     // embedding and the first layer's input norm in one kernel; every later norm comes out of a residual update
-        k_embed_norm<OT><<<R, 256, 0, st>>>(t, m->embed, W, emb_scale, sw_norm(m, m->L[m->runs[0].layer], 0), m->x, opA, wp);
+        pdl_launch(k_embed_norm<OT>, R, 256, 0, st, t, m->embed, W, emb_scale, sw_norm(m, m->L[m->runs[0].layer], 0), m->x, opA, wp);
         GTB_LAUNCHED();
     } else {
-        k_embed<OT><<<R, 256, 0, st>>>(t, m->embed, m->bigram, c.bigram_buckets, c.bigram_mul_prev, c.bigram_mul_cur, W, emb_scale,
+        pdl_launch(k_embed<OT>, R, 256, 0, st, t, m->embed, m->bigram, c.bigram_buckets, c.bigram_mul_prev, c.bigram_mul_cur, W, emb_scale,
                                        m->prenorm ? m->xs : m->x, c.loop_times > 0 ? m->x0 : nullptr, first_reads_x ? opA : (OT*)nullptr, wp);
         GTB_LAUNCHED();
         if (m->sandwich) {
-            k_norm_rows<OT><<<R, 256, 0, st>>>(m->x, W, sw_norm(m, m->L[m->runs[0].layer], 0), nullptr, opA, wp, 1.0f);
+            pdl_launch(k_norm_rows<OT>, R, 256, 0, st, m->x, W, sw_norm(m, m->L[m->runs[0].layer], 0), nullptr, opA, wp, 1.0f);
             GTB_LAUNCHED();
         }
     }
@@ -1386,7 +1386,7 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
         }
         x_in_opA = false;
         if (run.enters_pass) {
-            k_concat2<OT><<<R, 256, 0, st>>>(m->x, m->x0, W, opL, pad64(2 * W));
+            pdl_launch(k_concat2<OT>, R, 256, 0, st, m->x, m->x0, W, opL, pad64(2 * W));
             GTB_LAUNCHED();
             int rc = product<OT>(m, opL, pad64(2 * W), m->loop_in, pad64(2 * W), m->x, W, R, W, pad64(2 * W), m->loop_step + (size_t)run.pass * W, 0);
             if (rc) return rc;
@@ -1394,23 +1394,23 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
         OT* ob = l.ff > 0 ? opB : nullptr;
         const bool nc_fused = c.taps > 0 && c.taps <= 8 && m->fused_norm && R >= 32;     // few rows: two kernels with channel-wide grids are quicker
         if (nc_fused) {
-            k_norm_canon<OT><<<R, 256, 0, st>>>(t, m->x, W, c.eps, l.d_gain, c.taps, l.canon_a, l.ff > 0 ? l.canon_b : nullptr, run.tail, m->h, opA, ob, wp);
+            pdl_launch(k_norm_canon<OT>, R, 256, 0, st, t, m->x, W, c.eps, l.d_gain, c.taps, l.canon_a, l.ff > 0 ? l.canon_b : nullptr, run.tail, m->h, opA, ob, wp);
             GTB_LAUNCHED();
         } else {
-            k_rmsnorm_scalar<float><<<R, 256, 0, st>>>(m->x, W, c.eps, l.d_gain, nullptr, m->h, W);
+            pdl_launch(k_rmsnorm_scalar<float>, R, 256, 0, st, m->x, W, c.eps, l.d_gain, nullptr, m->h, W);
             GTB_LAUNCHED();
         }
         if (c.taps > 0) {
             if (!nc_fused) {
-                k_canon<OT><<<dim3(R, (W + 255) / 256), 256, 0, st>>>(t, m->h, W, c.taps, l.canon_a, l.ff > 0 ? l.canon_b : nullptr, run.tail, opA, ob, wp);
+                pdl_launch(k_canon<OT>, dim3(R, (W + 255) / 256), 256, 0, st, t, m->h, W, c.taps, l.canon_a, l.ff > 0 ? l.canon_b : nullptr, run.tail, opA, ob, wp);
                 GTB_LAUNCHED();
             }
             if (c.taps > 1) {
-                k_canon_tail<<<dim3(S, (W + 255) / 256), 256, 0, st>>>(t, m->h, W, W, c.taps, run.tail);
+                pdl_launch(k_canon_tail, dim3(S, (W + 255) / 256), 256, 0, st, t, m->h, W, W, c.taps, run.tail);
                 GTB_LAUNCHED();
             }
         } else {
-            k_copy_operand<OT><<<R, 256, 0, st>>>(m->h, W, opA, ob, wp);
+            pdl_launch(k_copy_operand<OT>, R, 256, 0, st, m->h, W, opA, ob, wp);
             GTB_LAUNCHED();
         }
         int rc = product<OT>(m, opA, wp, l.w_mix, wp, m->P, l.n1, R, l.n1, wp, nullptr, 0);
@@ -1432,7 +1432,7 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
             const BranchW& b = l.br[bi];
             if (b.d.kind == GTB_MIX_SIGMOID_ATTN) {
                 const AttnBranch a = attn_args(m, b);
-                k_attn_prep<OT><<<dim3(R, (a.heads + 2 * a.kv_heads + 3) / 4), 128, 0, st>>>(t, a, m->P, l.n1, (OT*)run.kc[bi], (OT*)run.vc[bi]);
+                pdl_launch(k_attn_prep<OT>, dim3(R, (a.heads + 2 * a.kv_heads + 3) / 4), 128, 0, st, t, a, m->P, l.n1, (OT*)run.kc[bi], (OT*)run.vc[bi]);
                 GTB_LAUNCHED();
                 int done = -1;
                 if (portions && sizeof(OT) == 2 && a.dim <= 128 && a.vdim <= 128)
@@ -1441,14 +1441,14 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
                 if (done < 0 && !portions && m->attn_splits > 1 && R <= SPLIT_MAX_ROWS) {
                     // (a group-major variant -- one CTA scoring a key for all query heads of its K/V head -- was measured slower at 32 heads
                     // and 8 splits: 8x fewer CTAs on a latency-bound step)
-                    k_sigattn_split<OT><<<dim3(R, a.heads, m->attn_splits), 128, (a.dim + 128) * sizeof(float), st>>>(t, a, m->P, l.n1, (const OT*)run.kc[bi], (const OT*)run.vc[bi], m->attn_part, R);
+                    pdl_launch(k_sigattn_split<OT>, dim3(R, a.heads, m->attn_splits), 128, (a.dim + 128) * sizeof(float), st, t, a, m->P, l.n1, (const OT*)run.kc[bi], (const OT*)run.vc[bi], m->attn_part, R);
                     GTB_LAUNCHED();
-                    k_sigattn_join<OT><<<dim3(R, (a.heads * a.vdim + 255) / 256), 256, 0, st>>>(a, m->attn_part, R, m->attn_splits, opC, l.kout_p);
+                    pdl_launch(k_sigattn_join<OT>, dim3(R, (a.heads * a.vdim + 255) / 256), 256, 0, st, a, m->attn_part, R, m->attn_splits, opC, l.kout_p);
                     GTB_LAUNCHED();
                     done = 0;
                 }
                 if (done < 0) {
-                    k_sigattn<OT><<<dim3(R, a.heads), 128, (a.dim + 128) * sizeof(float), st>>>(t, a, m->P, l.n1, (const OT*)run.kc[bi], (const OT*)run.vc[bi], opC, l.kout_p);
+                    pdl_launch(k_sigattn<OT>, dim3(R, a.heads), 128, (a.dim + 128) * sizeof(float), st, t, a, m->P, l.n1, (const OT*)run.kc[bi], (const OT*)run.vc[bi], opC, l.kout_p);
                     GTB_LAUNCHED();
                 }
             } else {
@@ -1458,7 +1458,7 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
         }
         if (l.ff > 0 && !ff_done) {
             const size_t n = (size_t)R * l.ff;
-            k_geglu<OT><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(m->G, l.ff, opC, l.kout_p, l.kout - l.ff, R, l.gu_inter ? 1 : 0);
+            pdl_launch(k_geglu<OT>, (unsigned)((n + 255) / 256), 256, 0, st, m->G, l.ff, opC, l.kout_p, l.kout - l.ff, R, l.gu_inter ? 1 : 0);
             GTB_LAUNCHED();
         }
         rc = product<OT>(m, opC, l.kout_p, l.w_out, l.kout_p, m->x, W, R, W, l.kout_p, nullptr, 1);
@@ -1470,28 +1470,28 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
     }
     if (n_want > 0) {
         float ls = c.logit_scale != 0.0f ? c.logit_scale : 1.0f;        // what is left of the logit scale for the logits themselves
-        if (c.final_norm == 5) k_rmsnorm_weight<OT><<<n_want, 256, 0, st>>>(m->x, W, c.eps, m->final_gain, 0, d_want, opH, wp);
+        if (c.final_norm == 5) pdl_launch(k_rmsnorm_weight<OT>, n_want, 256, 0, st, m->x, W, c.eps, m->final_gain, 0, d_want, opH, wp);
         else if (c.final_norm >= 3) {
             NormArgs fn{};
             fn.kind = GTB_NORM_LAYER; fn.w = m->final_gain; fn.b = m->final_b; fn.eps = c.eps;
-            k_norm_rows<OT><<<n_want, 256, 0, st>>>(m->x, W, fn, d_want, opH, wp, ls);      // the product is linear: the scale rides on its operand
+            pdl_launch(k_norm_rows<OT>, n_want, 256, 0, st, m->x, W, fn, d_want, opH, wp, ls);      // the product is linear: the scale rides on its operand
             ls = 1.0f;
         } else if (c.final_norm == 2) {
             NormArgs fn{};
             fn.kind = GTB_NORM_DYT; fn.w = m->final_gain; fn.b = m->final_b; fn.alpha = m->final_a;
-            k_dyt_rows<OT><<<n_want, 256, 0, st>>>(m->x, W, fn, d_want, opH, wp);
-        } else if (c.final_norm) k_rmsnorm_weight<OT><<<n_want, 256, 0, st>>>(m->x, W, c.eps, m->final_gain, 1, d_want, opH, wp);
-        else k_rmsnorm_scalar<OT><<<n_want, 256, 0, st>>>(m->x, W, c.eps, m->final_gain, d_want, opH, wp);
+            pdl_launch(k_dyt_rows<OT>, n_want, 256, 0, st, m->x, W, fn, d_want, opH, wp);
+        } else if (c.final_norm) pdl_launch(k_rmsnorm_weight<OT>, n_want, 256, 0, st, m->x, W, c.eps, m->final_gain, 1, d_want, opH, wp);
+        else pdl_launch(k_rmsnorm_scalar<OT>, n_want, 256, 0, st, m->x, W, c.eps, m->final_gain, d_want, opH, wp);
         GTB_LAUNCHED();
         int rc = product<OT>(m, opH, wp, m->head, wp, m->logits, c.vocab, n_want, c.vocab, wp, nullptr, 0);
         if (rc) return rc;
         if (c.logit_softcap > 0.0f || ls != 1.0f) {
             const size_t n = (size_t)n_want * c.vocab;
-            k_logits_post<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(m->logits, n, ls, c.logit_softcap);
+            pdl_launch(k_logits_post, (unsigned)((n + 255) / 256), 256, 0, st, m->logits, n, ls, c.logit_softcap);
             GTB_LAUNCHED();
         }
     }
-    k_commit<<<(S + 127) / 128, 128, 0, st>>>(t, S);
+    pdl_launch(k_commit, (S + 127) / 128, 128, 0, st, t, S);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -2427,7 +2427,7 @@ static int step_impl(gtb_seq_t m, int n_seg, const int32_t* seg_slot, const int3
             GTB_CUDA(cudaMemcpyAsync(m->d_tab + n_ints, m->h_tab + n_ints, nw * sizeof(int), cudaMemcpyHostToDevice, st));
             PassTables ta = t;
             ta.seg_slot = m->d_tab + n_ints;
-            k_argmax_rows<<<nw, 1024, 0, st>>>(m->logits, c.vocab, ta, -1, m->d_hist, 1, 0);
+            pdl_launch(k_argmax_rows, nw, 1024, 0, st, m->logits, c.vocab, ta, -1, m->d_hist, 1, 0);
             GTB_LAUNCHED();
             std::vector<int> got(nw);
             GTB_CUDA(cudaMemcpyAsync(got.data(), m->d_hist, nw * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -2493,7 +2493,7 @@ int gtb_seq_decode(gtb_seq_t m, int n, const int32_t* slots, int n_steps, int eo
     auto one = [&]() -> int {
         int rc = c.mode == GTB_SEQ_F32 ? run_pass<float>(m, t, n, n, true, n, d_want) : run_pass<bf16>(m, t, n, n, true, n, d_want);
         if (rc) return rc;
-        k_argmax_rows<<<n, 1024, 0, st>>>(m->logits, c.vocab, t, eos_id, m->d_hist, 1, 0);
+        pdl_launch(k_argmax_rows, n, 1024, 0, st, m->logits, c.vocab, t, eos_id, m->d_hist, 1, 0);
         GTB_LAUNCHED();
         return GTB_OK;
     };

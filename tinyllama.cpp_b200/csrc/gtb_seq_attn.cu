@@ -104,6 +104,7 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
     using Cfg = AtCfg<DP, VP>;
     constexpr int KT = AT_KT, AT_STAGES = Cfg::STAGES;
     extern __shared__ unsigned char smem_raw[];
+    pdl_wait();
     // the CTA's tile: 128 rows of a segment.  Tiles are the slow grid dimension and a segment's last tiles, which sweep the most keys, come
     // first: every unit's longest tiles start before any shorter one
     int seg = -1, q0 = 0;
@@ -152,6 +153,7 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
     __syncthreads();
     tc_fence_after();
     const uint32_t tm = *tmem_slot;
+    pdl_trigger();                  // (behind the TMEM allocation)
 
     if (warp == 4) {
         if (lane == 0) {            // ---------------- TMA producer
@@ -413,7 +415,7 @@ static int launch(SeqGemmPlan* p, const AttnTc& a, int n_tiles) {
     if (rc) return rc;
     static bool attr = false;
     if (!attr) { GTB_CUDA(cudaFuncSetAttribute(k_attn_tc<DP, VP, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM)); attr = true; }
-    k_attn_tc<DP, VP, SIG><<<dim3(a.heads * a.maps, n_tiles), AT_THREADS, Cfg::SMEM, ctx().stream>>>(tk, tv, a, p->d_status);
+    pdl_launch(k_attn_tc<DP, VP, SIG>, dim3(a.heads * a.maps, n_tiles), AT_THREADS, Cfg::SMEM, ctx().stream, tk, tv, a, p->d_status);
     GTB_LAUNCHED();
     return GTB_OK;
 }

@@ -130,6 +130,7 @@ k_seq_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger_and_wait();        // (behind the TMEM allocation)
 
     if (warp == 0) {
         if (lane == 0) {        // ---------------- TMA producer
@@ -367,11 +368,21 @@ k_seq_skinny(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();                 // (behind the TMEM allocation)
+    if (threadIdx.x != 0) pdl_wait();      // the producer thread waits behind its first loads of W
 
     if (warp == 0) {
         if (lane == 0) {        // ---------------- TMA producer
-            uint32_t s = 0, ph = 0;
-            for (int kb = kb0; kb < kb1; kb++) {
+            // W does not depend on the kernels before: its first stages are on their way while those finish
+            const int pre = min(ST, kb1 - kb0);
+            for (int i = 0; i < pre; i++) {
+                mbar_expect_tx(bar_full(i), Cfg::STAGE_BYTES);
+                tma_load_2d(smem_base + i * Cfg::STAGE_BYTES, &tmW, bar_full(i), (kb0 + i) % ep.w_blocks * SQ_BK, n0);
+            }
+            pdl_wait();
+            for (int i = 0; i < pre; i++) tma_load_2d(smem_base + i * Cfg::STAGE_BYTES + Cfg::W_BYTES, &tmA, bar_full(i), (kb0 + i) * SQ_BK, m0);
+            uint32_t s = pre % ST, ph = pre == ST ? 1 : 0;
+            for (int kb = kb0 + pre; kb < kb1; kb++) {
                 if (!sq_wait(bar_empty(s), ph ^ 1, abort_flag)) break;
                 mbar_expect_tx(bar_full(s), Cfg::STAGE_BYTES);
                 const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES;
@@ -524,7 +535,7 @@ static int launch(SeqGemmPlan* p, const CUtensorMap& ta, const CUtensorMap& tb, 
     constexpr int TM = SWAP ? BN : SQ_BM, TN = SWAP ? SQ_BM : BN;
     const int n_tiles = ((M + TM - 1) / TM) * ((N + TN - 1) / TN);
     const int grid = n_tiles < ctx().sm_count ? n_tiles : ctx().sm_count;
-    k_seq_gemm<BN, EPI, SWAP><<<grid, SQ_THREADS, Cfg::SMEM, ctx().stream>>>(ta, tb, M, N, K, ep);
+    pdl_launch(k_seq_gemm<BN, EPI, SWAP>, grid, SQ_THREADS, Cfg::SMEM, ctx().stream, ta, tb, M, N, K, ep);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -536,17 +547,7 @@ static int launch_skinny(bool& attr, const CUtensorMap& tw, const CUtensorMap& t
         GTB_CUDA(cudaFuncSetAttribute(k_seq_skinny<MT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
         attr = true;
     }
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3((N + 127) / 128 * cs, (M + MT - 1) / MT);
-    lc.blockDim = dim3(SK_THREADS);
-    lc.dynamicSmemBytes = Cfg::SMEM;
-    lc.stream = ctx().stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    GTB_CUDA(cudaLaunchKernelEx(&lc, k_seq_skinny<MT, EPI>, tw, ta, M, N, K, cs, ep));
+    pdl_launch_cluster(cs, k_seq_skinny<MT, EPI>, dim3((N + 127) / 128 * cs, (M + MT - 1) / MT), SK_THREADS, Cfg::SMEM, ctx().stream, tw, ta, M, N, K, cs, ep);
     GTB_LAUNCHED();
     return GTB_OK;
 }

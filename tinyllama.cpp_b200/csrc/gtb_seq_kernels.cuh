@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "gtb_tc.cuh"
+
 namespace gtb {
 namespace seq {
 
@@ -106,6 +108,7 @@ __device__ __forceinline__ float gelu_erf(float z) { return 0.5f * z * (1.0f + e
 // ------------------------------------------------------------------------------------------------ plan / commit
 // row tables of a pass from the slots' device-side state.  from_pending: rows take their token from the slot (decode loop).
 __global__ void k_plan(PassTables t, int R, int from_pending) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= R) return;
     const int s = t.row_seg[r], slot = t.seg_slot[s], row0 = t.seg_row0[s];
@@ -116,6 +119,7 @@ __global__ void k_plan(PassTables t, int R, int from_pending) {
     t.row_prev[r] = (r > row0) ? (from_pending ? st.pending : t.tok[r - 1]) : (pos == 0 ? -1 : st.prev);
 }
 __global__ void k_commit(PassTables t, int S) {
+    pdl_trigger_and_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= S) return;
     SlotState& st = t.slots[t.seg_slot[s]];
@@ -130,6 +134,7 @@ __global__ void k_commit(PassTables t, int S) {
 template <typename OT>
 __global__ void k_embed(PassTables t, const bf16* __restrict__ embed, const bf16* __restrict__ bigram, int buckets, int mul_prev,
                         int mul_cur, int width, float scale, float* __restrict__ x, float* __restrict__ x0, OT* __restrict__ op, int ld_op) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x;
     const int tok = t.tok[r], prev = t.row_prev[r];
     long long row = buckets;
@@ -148,6 +153,7 @@ __global__ void k_embed(PassTables t, const bf16* __restrict__ embed, const bf16
 template <typename OUT>
 __global__ void k_rmsnorm_scalar(const float* __restrict__ x, int width, float eps, const float* __restrict__ g, const int* __restrict__ rows,
                                  OUT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     __shared__ float red[33];
     const int o = blockIdx.x, r = rows ? rows[o] : o;
     const float* xr = x + (size_t)r * width;
@@ -164,6 +170,7 @@ __global__ void k_rmsnorm_scalar(const float* __restrict__ x, int width, float e
 template <typename OT>
 __global__ void k_canon(PassTables t, const float* __restrict__ h, int width, int taps, const bf16* __restrict__ wa, const bf16* __restrict__ wb,
                         const float* __restrict__ tail, OT* __restrict__ out_a, OT* __restrict__ out_b, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x;
     const int s = t.row_seg[r], row0 = t.seg_row0[s], slot = t.seg_slot[s];
     const float* tl = tail + (size_t)slot * (taps - 1) * width;
@@ -187,6 +194,7 @@ template <typename OT>
 __global__ void __launch_bounds__(256) k_norm_canon(PassTables t, const float* __restrict__ x, int width, float eps, const float* __restrict__ g, int taps,
                                                     const bf16* __restrict__ wa, const bf16* __restrict__ wb, const float* __restrict__ tail,
                                                     float* __restrict__ h, OT* __restrict__ out_a, OT* __restrict__ out_b, int ld_out) {
+    pdl_trigger_and_wait();
     __shared__ float inv[32];
     const int r = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int s = t.row_seg[r], row0 = t.seg_row0[s], slot = t.seg_slot[s];
@@ -219,6 +227,7 @@ __global__ void __launch_bounds__(256) k_norm_canon(PassTables t, const float* _
 // no convolution configured: the operand is h itself
 template <typename OT>
 __global__ void k_copy_operand(const float* __restrict__ h, int width, OT* __restrict__ out_a, OT* __restrict__ out_b, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x;
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         const OT v = cvt<OT>(h[(size_t)r * width + c]);
@@ -229,6 +238,7 @@ __global__ void k_copy_operand(const float* __restrict__ h, int width, OT* __res
 // history <- the last taps - 1 values of h of each segment's sequence.  One thread per channel walks k upwards: entry k is written
 // after every entry it is read for (k + len > k).
 __global__ void k_canon_tail(PassTables t, const float* __restrict__ h, int ldh, int width, int taps, float* __restrict__ tail) {
+    pdl_trigger_and_wait();
     const int s = blockIdx.x;
     const int row0 = t.seg_row0[s], len = t.seg_len[s], slot = t.seg_slot[s];
     if (t.slots[slot].stopped) return;
@@ -246,6 +256,7 @@ constexpr int SG_BM = 64, SG_BN = 64, SG_BK = 16;
 template <typename AT>
 __global__ void __launch_bounds__(256) k_gemm_simt(const AT* __restrict__ A, int lda, const bf16* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
                                                    int M, int N, int K, const float* __restrict__ bias, int accumulate) {
+    pdl_trigger_and_wait();
     __shared__ float sa[SG_BK][SG_BM + 4];
     __shared__ float sw[SG_BK][SG_BN + 4];
     const int m0 = blockIdx.y * SG_BM, n0 = blockIdx.x * SG_BN;
@@ -293,6 +304,7 @@ __global__ void __launch_bounds__(256) k_gemm_simt(const AT* __restrict__ A, int
 // come first so that the accumulator meets them before the large sums.  300 rows x 4864 x 1024: split 4 us + product 22 us against 240 us on
 // FFMA; two-layer logits 1.5e-6 from float64 against 1.9e-6.
 __global__ void __launch_bounds__(256) k_split3(const float* __restrict__ A, int lda, int K, bf16* __restrict__ out) {
+    pdl_trigger_and_wait();
     const float* a = A + (size_t)blockIdx.x * lda;
     uint2* o = reinterpret_cast<uint2*>(out + (size_t)blockIdx.x * 3 * K);
     for (int i = threadIdx.x; i < K / 4; i += blockDim.x) {
@@ -319,11 +331,11 @@ __global__ void __launch_bounds__(256) k_split3(const float* __restrict__ A, int
 // rows of A come through L1 as 16-byte loads too), the lanes' partial sums meet in a shuffle reduction and the warps' in shared memory.
 template <typename AT> __device__ __forceinline__ void load8(const AT* p, float (&v)[8]);
 template <> __device__ __forceinline__ void load8<float>(const float* p, float (&v)[8]) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p + 4));
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 template <> __device__ __forceinline__ void load8<bf16>(const bf16* p, float (&v)[8]) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 a = *reinterpret_cast<const uint4*>(p);
     const uint32_t w[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
     for (int i = 0; i < 4; i++) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
@@ -341,13 +353,22 @@ __global__ void __launch_bounds__(256) k_gemv_rows(const AT* __restrict__ A, int
     for (int m = 0; m < MR; m++)
 #pragma unroll
         for (int c = 0; c < NC; c++) acc[m][c] = 0.0f;
-    // K % 64 == 0 and every row is 16-byte aligned: steps of 8 elements never straddle the end
-#pragma unroll 2
-    for (int k = (warp * 32 + lane) * 8; k < K; k += 2048) {
-        uint4 wv[NC];
+    // K % 64 == 0 and every row is 16-byte aligned: steps of 8 elements never straddle the end.  The weights do not depend on the kernels before:
+    // the first step's loads are in flight while those finish, a step's loads while the step before is summed
+    int k = (warp * 32 + lane) * 8;
+    uint4 wn[NC];
+    auto fetch = [&](int kk) {
 #pragma unroll
         for (int c = 0; c < NC; c++)
-            wv[c] = (n0 + c < N) ? __ldg(reinterpret_cast<const uint4*>(W + (size_t)(n0 + c) * ldw + k)) : make_uint4(0, 0, 0, 0);
+            wn[c] = (n0 + c < N) ? __ldg(reinterpret_cast<const uint4*>(W + (size_t)(n0 + c) * ldw + kk)) : make_uint4(0, 0, 0, 0);
+    };
+    if (k < K) fetch(k);
+    pdl_trigger_and_wait();
+    for (; k < K; k += 2048) {
+        uint4 wv[NC];
+#pragma unroll
+        for (int c = 0; c < NC; c++) wv[c] = wn[c];
+        if (k + 2048 < K) fetch(k + 2048);
 #pragma unroll
         for (int m = 0; m < MR; m++) {
             if (m >= M) break;
@@ -402,6 +423,7 @@ struct AttnBranch {
 // q (and k) to unit RMS per head in place; k, v of every row appended to the slot's cache [n_slots][max_ctx][kv_heads * dim|vdim].
 template <typename OT>
 __global__ void k_attn_prep(PassTables t, AttnBranch b, float* __restrict__ P, int ldp, OT* __restrict__ kc, OT* __restrict__ vc) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int slot = t.seg_slot[t.row_seg[r]], pos = t.row_pos[r];
     float* p = P + (size_t)r * ldp;
@@ -435,6 +457,7 @@ __global__ void k_attn_prep(PassTables t, AttnBranch b, float* __restrict__ P, i
 template <typename OT>
 __global__ void __launch_bounds__(128) k_sigattn(PassTables t, AttnBranch b, const float* __restrict__ P, int ldp, const OT* __restrict__ kc,
                                                  const OT* __restrict__ vc, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     extern __shared__ float sm[];
     float* sq = sm;                 // [dim]
     float* swt = sm + b.dim;        // [blockDim.x]
@@ -483,6 +506,7 @@ __global__ void __launch_bounds__(128) k_sigattn(PassTables t, AttnBranch b, con
 template <typename OT>
 __global__ void __launch_bounds__(128) k_sigattn_split(PassTables t, AttnBranch b, const float* __restrict__ P, int ldp, const OT* __restrict__ kc,
                                                        const OT* __restrict__ vc, float* __restrict__ part, int R) {
+    pdl_trigger_and_wait();
     extern __shared__ float sm[];
     float* sq = sm;
     float* swt = sm + b.dim;
@@ -551,6 +575,7 @@ __global__ void __launch_bounds__(128) k_sigattn_split(PassTables t, AttnBranch 
 }
 template <typename OT>
 __global__ void k_sigattn_join(AttnBranch b, const float* __restrict__ part, int R, int splits, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, n = b.heads * b.vdim;
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < n; c += gridDim.y * blockDim.x) {
         float a = 0.0f;
@@ -576,6 +601,7 @@ struct RetBranch {
 // returns to the slot's state in HBM.  q and k are rotated (pairs i, i + rot_dims/2) and k scaled here.
 // raw o goes to O [R][heads * vdim] (fp32); normalisation and the gate follow in k_ret_post.
 __global__ void k_retention(PassTables t, RetBranch b, const float* __restrict__ P, int ldp, float* __restrict__ state, float* __restrict__ O, int vs) {
+    pdl_trigger_and_wait();
     extern __shared__ float sm[];
     const int s = blockIdx.x, h = blockIdx.y;
     const int slot = t.seg_slot[s], row0 = t.seg_row0[s], len = t.seg_len[s];
@@ -643,6 +669,7 @@ __global__ void k_retention(PassTables t, RetBranch b, const float* __restrict__
 // per (row, head): o / rms(o) (optional), * silu(gate) (optional), * out_scale -> operand of the out projection
 template <typename OT>
 __global__ void k_ret_post(RetBranch b, const float* __restrict__ O, const float* __restrict__ P, int ldp, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int h = blockIdx.y * nw + wid; h < b.heads; h += gridDim.y * nw) {
         const float* o = O + (size_t)r * (b.heads * b.vdim) + h * b.vdim;
@@ -666,6 +693,7 @@ __global__ void k_ret_post(RetBranch b, const float* __restrict__ O, const float
 // (interleaved) groups of 32 gate columns each followed by its 32 up columns.
 template <typename OT>
 __global__ void k_geglu(const float* __restrict__ G, int ff, OT* __restrict__ out, int ld_out, int a_off, int R, int interleaved) {
+    pdl_trigger_and_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)R * ff) return;
     const int r = (int)(i / ff), c = (int)(i % ff);
@@ -675,6 +703,7 @@ __global__ void k_geglu(const float* __restrict__ G, int ff, OT* __restrict__ ou
 // operand [x | x0] of the loop's entry projection
 template <typename OT>
 __global__ void k_concat2(const float* __restrict__ x, const float* __restrict__ x0, int width, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x;
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         out[(size_t)r * ld_out + c] = cvt<OT>(x[(size_t)r * width + c]);
@@ -687,15 +716,28 @@ __global__ void k_concat2(const float* __restrict__ x, const float* __restrict__
 // slot's pending token and lands in hist[row][step]; a slot that samples eos_id stops.
 __global__ void __launch_bounds__(1024) k_argmax_rows(const float* __restrict__ logits, int n, PassTables t, int eos_id, int* __restrict__ out,
                                                        int out_ld, int out_col) {
+    pdl_trigger_and_wait();
     __shared__ float sv[32];
     __shared__ int si[32];
     const int s = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const float* lg = logits + (size_t)s * n;
     float best = -INFINITY;
     int arg = 0x7fffffff;
-    for (int j = tid; j < n; j += blockDim.x) {
-        const float v = lg[j];
-        if (v > best) { best = v; arg = j; }
+    if (n % 4 == 0) {                       // ascending within a thread, so a strict comparison keeps its first maximum; four loads in flight
+        const float4* l4 = reinterpret_cast<const float4*>(lg);
+#pragma unroll 4
+        for (int j = tid; j < n / 4; j += blockDim.x) {
+            const float4 v = l4[j];
+            if (v.x > best) { best = v.x; arg = 4 * j; }
+            if (v.y > best) { best = v.y; arg = 4 * j + 1; }
+            if (v.z > best) { best = v.z; arg = 4 * j + 2; }
+            if (v.w > best) { best = v.w; arg = 4 * j + 3; }
+        }
+    } else {
+        for (int j = tid; j < n; j += blockDim.x) {
+            const float v = lg[j];
+            if (v > best) { best = v; arg = j; }
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -742,6 +784,7 @@ __device__ __forceinline__ bool ret_find_chunk(const PassTables& t, int S, int C
 }
 
 __global__ void k_ret_rotate(PassTables t, RetBranch b, float* __restrict__ P, int ldp) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x;
     float* p = P + (size_t)r * ldp;
     const float pos = (float)t.row_pos[r];
@@ -766,6 +809,7 @@ __global__ void k_ret_rotate(PassTables t, RetBranch b, float* __restrict__ P, i
 // accumulates 4 x 4 tiles of U from float4 reads (dp, vsp: dim and the slice width rounded up to 4, zero-filled).
 __global__ void __launch_bounds__(256) k_ret_chunk_kv(PassTables t, RetBranch b, const float* __restrict__ P, int ldp, int S, int C, int vs,
                                                       float* __restrict__ U) {
+    pdl_trigger_and_wait();
     extern __shared__ __align__(16) float sm[];
     int seg, c;
     if (!ret_find_chunk(t, S, C, blockIdx.x, seg, c)) return;
@@ -818,6 +862,7 @@ template <int V> __device__ __forceinline__ void rs_store(float* p, const float 
 // on their own; a batch's loads are issued before the dependent chain of multiply-adds starts
 template <int V>
 __global__ void __launch_bounds__(256) k_ret_scan(PassTables t, RetBranch b, int S, int C, float* __restrict__ U, float* __restrict__ state) {
+    pdl_trigger_and_wait();
     constexpr int NB = V == 4 ? 8 : 16;
     const int seg = blockIdx.x, h = blockIdx.y;
     const int e = (blockIdx.z * blockDim.x + threadIdx.x) * V;
@@ -855,6 +900,7 @@ __global__ void __launch_bounds__(256) k_ret_scan(PassTables t, RetBranch b, int
 // are one float4), v [C][vsp], aT [C keys][C rows] = g^(a-b) q_a.k_b for b <= a, s0 [dim][vsp].  Three products on 4 x 4 register tiles.
 __global__ void __launch_bounds__(256) k_ret_chunk_out(PassTables t, RetBranch b, const float* __restrict__ P, int ldp, int S, int C, int vs,
                                                        const float* __restrict__ Sb, float* __restrict__ O) {
+    pdl_trigger_and_wait();
     extern __shared__ __align__(16) float sm[];
     int seg, c;
     if (!ret_find_chunk(t, S, C, blockIdx.x, seg, c)) return;
@@ -968,6 +1014,7 @@ constexpr int RT_C = 64, RT_V = 128;      // rows per chunk, value channels per 
 
 // U [chunk][head][dim][vdim]; grid (chunks, heads, value slices), 256 threads.  Shared memory: k' [64][128], v [64][128] (zeros beyond the head)
 __global__ void __launch_bounds__(256) k_ret_kv_wide(PassTables t, RetBranch b, const float* __restrict__ P, int ldp, int S, float* __restrict__ U) {
+    pdl_trigger_and_wait();
     extern __shared__ __align__(16) float sm[];
     float* sk = sm;
     float* sv = sm + RT_C * 128;
@@ -1026,6 +1073,7 @@ __global__ void __launch_bounds__(256) k_ret_kv_wide(PassTables t, RetBranch b, 
 constexpr int RT_CP = RT_C + 4;
 constexpr size_t RT_OUT_SMEM = (2 * 128 * RT_CP + RT_C * RT_C + RT_C + 4) * sizeof(float);
 __global__ void __launch_bounds__(256, 2) k_ret_out_wide(PassTables t, RetBranch b, const float* __restrict__ P, int ldp, int S, const float* __restrict__ Sb, float* __restrict__ O) {
+    pdl_trigger_and_wait();
     extern __shared__ __align__(16) float sm[];
     float* sq = sm;                        // [128][RT_CP]
     float* sk = sq + 128 * RT_CP;          // [128][RT_CP]; then [2][32][128]
@@ -1193,6 +1241,7 @@ __device__ __forceinline__ void sa_cp16(uint32_t dst, const void* src, bool vali
 template <int DP, int VP, int HPC>
 __global__ void __launch_bounds__(128 * HPC) k_sigattn_mma(PassTables t, AttnBranch b, int S, const float* __restrict__ P, int ldp, const bf16* __restrict__ kc,
                                                      const bf16* __restrict__ vc, bf16* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     constexpr int LQ = DP + 8, LV = VP + 8;
     extern __shared__ __align__(16) unsigned char sa_raw[];
     bf16* sq = reinterpret_cast<bf16*>(sa_raw);          // [HPC][64][LQ]: the CTA's query heads share one K/V head

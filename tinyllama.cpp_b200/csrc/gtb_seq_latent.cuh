@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(256, NSM <= 4 ? 3 : 2) k_hc_step(float* __rest
                                                  const int* __restrict__ pair_dst, int top, const float* __restrict__ hc_prev,
                                                  const float* __restrict__ in_next, NormArgs nrm, OT* __restrict__ op, int ld_op,
                                                  float* __restrict__ xsum) {
+    pdl_trigger_and_wait();
     __shared__ float red[33];
     __shared__ float sh[2 * HC_MAX + HC_MAX * HC_MAX + HC_MAX];
     __shared__ int sdst[PN_MAX_TOP];
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(256, NSM <= 4 ? 3 : 2) k_hc_step(float* __rest
 template <typename OUT>
 __global__ void __launch_bounds__(256) k_dyt_rows(const float* __restrict__ x, int width, NormArgs nrm, const int* __restrict__ rows,
                                                   OUT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int o = blockIdx.x, r = rows ? rows[o] : o;
     const float a = nrm.alpha[0];
     for (int c = threadIdx.x; c < width; c += blockDim.x)
@@ -150,6 +152,7 @@ __global__ void __launch_bounds__(256) k_dyt_rows(const float* __restrict__ x, i
 
 // logits <- scale * logits, then cap * tanh(. / cap) when cap > 0
 __global__ void k_logits_post(float* __restrict__ v, size_t n, float scale, float cap) {
+    pdl_trigger_and_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float z = scale * v[i];
@@ -181,6 +184,7 @@ __device__ __forceinline__ void rot_pair(const LatAttn& b, int pr, int& i0, int&
 template <typename OT>
 __global__ void __launch_bounds__(128) k_lat_prep(PassTables t, LatAttn b, const float* __restrict__ P, int ldp, OT* __restrict__ cache,
                                                   OT* __restrict__ opq, int ld_q) {
+    pdl_trigger_and_wait();
     __shared__ float red[33];
     const int r = blockIdx.x;
     const int slot = t.seg_slot[t.row_seg[r]], pos = t.row_pos[r];
@@ -216,6 +220,7 @@ __global__ void __launch_bounds__(128) k_lat_prep(PassTables t, LatAttn b, const
 // Prompt portions: the heads' queries with their rotated part turned to the row's position: QR [R][ld_qr] = heads x (plain | rotated).
 // Q may be QR itself (in place).
 __global__ void __launch_bounds__(128) k_lat_qrot(PassTables t, LatAttn b, const float* Q, int ldq, int q0, float* QR, int ld_qr) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, hd = b.dim + b.rope;
     const float fpos = (float)t.row_pos[r];
     const float* q = Q + (size_t)r * ldq + q0;
@@ -242,6 +247,7 @@ __global__ void __launch_bounds__(128) k_lat_qrot(PassTables t, LatAttn b, const
 // Kx [n_slots][max_ctx][heads][dim + rope] <- [plain key | the cached rotated part], Vx [n_slots][max_ctx][heads][vdim].
 __global__ void __launch_bounds__(256) k_lat_pack(LatAttn b, const float* __restrict__ X, int n, int slot, int lo, const bf16* __restrict__ cache,
                                                   bf16* __restrict__ Kx, bf16* __restrict__ Vx) {
+    pdl_trigger_and_wait();
     const int j = blockIdx.x, hd = b.dim + b.rope;
     const size_t row = (size_t)slot * b.max_ctx + lo + j;
     const float* x = X + (size_t)j * b.heads * (b.dim + b.vdim);
@@ -262,6 +268,7 @@ __global__ void __launch_bounds__(256) k_lat_pack(LatAttn b, const float* __rest
 // the plain entries, a lane takes four adjacent columns (one 8-byte load per entry), the warps' sums meet in shared memory.
 __global__ void __launch_bounds__(128) k_lat_qabs(PassTables t, LatAttn b, const float* __restrict__ Q, int ldq, int q0, const bf16* __restrict__ uk, int ld_uk,
                                                   float* __restrict__ QA) {
+    pdl_trigger_and_wait();
     extern __shared__ float sq[];             // [dim + rope], then [4][128] partial sums
     const int r = blockIdx.x, h = blockIdx.y, hd = b.dim + b.rope;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -317,6 +324,7 @@ __global__ void __launch_bounds__(128) k_lat_qabs(PassTables t, LatAttn b, const
 template <int VPW>
 __global__ void __launch_bounds__(128) k_lat_dec_mma(PassTables t, SoftAttn b, const float* __restrict__ QA, int ldqa, const bf16* __restrict__ cache,
                                                      float* __restrict__ part, int R) {
+    pdl_trigger_and_wait();
     constexpr int TK = 64;
     extern __shared__ __align__(16) unsigned char ld_raw[];
     const int D = b.dim, DP = (D + 15) & ~15, LK = DP + 8, LP = TK + 8;
@@ -472,6 +480,7 @@ __global__ void __launch_bounds__(128) k_lat_dec_mma(PassTables t, SoftAttn b, c
 template <typename OT>
 __global__ void __launch_bounds__(256) k_lat_vup(LatAttn b, const OT* __restrict__ OL, int ld_ol, const bf16* __restrict__ uv, int ld_uv,
                                                  const float* __restrict__ P, int ldp, int gate, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n = b.heads * b.vdim;
     const bool vec = b.rank % 8 == 0 && ld_ol % 8 == 0 && ld_uv % 8 == 0;
@@ -509,6 +518,7 @@ __global__ void __launch_bounds__(256) k_lat_vup(LatAttn b, const OT* __restrict
 // Shared memory: n_exp floats.
 __global__ void __launch_bounds__(32) k_moe_route_sigmoid(const float* __restrict__ Z, int ldz, int n_exp, int top, int* __restrict__ sel_idx,
                                                           float* __restrict__ sel_w, float* __restrict__ shared_w) {
+    pdl_trigger_and_wait();
     extern __shared__ float ch[];
     const int r = blockIdx.x, lane = threadIdx.x;
     const float* z = Z + (size_t)r * ldz;
@@ -547,6 +557,7 @@ template <typename OT>
 __global__ void __launch_bounds__(256) k_moe_gu_rows(const OT* __restrict__ X, int ldx, int K, const bf16* __restrict__ w_gu, int ldw, int ff, int kfp,
                                                      int inter, int top, const int* __restrict__ sel_idx, const float* __restrict__ sel_w,
                                                      OT* __restrict__ act) {
+    pdl_trigger_and_wait();
     const int pair = blockIdx.x, r = pair / top, e = sel_idx[pair];
     const float wt = sel_w[pair];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -566,6 +577,7 @@ __global__ void __launch_bounds__(256) k_moe_gu_rows(const OT* __restrict__ X, i
 // (grid: rows x column groups; few rows spread their columns over many CTAs)
 template <typename OT>
 __global__ void k_swiglu_rows(const float* __restrict__ G, int ff, int inter, const float* __restrict__ row_w, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x;
     const float wt = row_w ? row_w[r] : 1.0f;
     const float* g = G + (size_t)r * 2 * ff;

@@ -47,6 +47,7 @@ __device__ __forceinline__ void store4(bf16* p, float a, float b, float c, float
 template <typename OUT>
 __global__ void __launch_bounds__(256) k_rmsnorm_weight(const float* __restrict__ x, int width, float eps, const float* __restrict__ w, int one_plus,
                                                         const int* __restrict__ rows, OUT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     __shared__ float red[33];
     const int o = blockIdx.x, r = rows ? rows[o] : o;
     const float* xr = x + (size_t)r * width;
@@ -89,6 +90,7 @@ __device__ __forceinline__ void route_row(const float* __restrict__ z, int n_out
 // rows of router logits Z -> choices; shared memory: 2 n_out floats
 __global__ void __launch_bounds__(32) k_moe_route(const float* __restrict__ Z, int ldz, int n_out, const float* __restrict__ corr, int top,
                                                   int* __restrict__ sel_idx, float* __restrict__ sel_w) {
+    pdl_trigger_and_wait();
     extern __shared__ float sm[];
     const int r = blockIdx.x;
     route_row(Z + (size_t)r * ldz, n_out, corr, top, sel_idx + (size_t)r * top, sel_w + (size_t)r * top, sm, sm + n_out, threadIdx.x);
@@ -137,6 +139,7 @@ __global__ void __launch_bounds__(256) k_postnorm_add(const float* __restrict__ 
                                                       const int* __restrict__ sel_idx, const float* __restrict__ sel_w, int top, int n_experts,
                                                       const float* __restrict__ Yg, const int* __restrict__ pair_dst,
                                                       float* __restrict__ x, OT* __restrict__ op, int ld_op, RouteNext rn) {
+    pdl_trigger_and_wait();
     __shared__ float red[33];
     __shared__ int sdst[PN_MAX_TOP];
     extern __shared__ float srt[];       // routing: the new stream row [width], logits [n_out], two work arrays [n_out]
@@ -218,6 +221,7 @@ __device__ __forceinline__ float gru_candidate(float u) { return u >= 0.0f ? u +
 template <typename OT>
 __global__ void __launch_bounds__(128) k_mingru(PassTables t, GruBranch b, const float* __restrict__ P, int ldp, float* __restrict__ state,
                                                 OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int s = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
     if (c >= b.width) return;
     const int slot = t.seg_slot[s], row0 = t.seg_row0[s], len = t.seg_len[s];
@@ -256,6 +260,7 @@ __device__ __forceinline__ bool gru_find_chunk(const PassTables& t, int S, int C
     return false;
 }
 __global__ void __launch_bounds__(128) k_mingru_chunk(PassTables t, GruBranch b, const float* __restrict__ P, int ldp, int S, int C, float* __restrict__ AB) {
+    pdl_trigger_and_wait();
     int seg, ck, first;
     if (!gru_find_chunk(t, S, C, blockIdx.x, seg, ck, first)) return;
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
@@ -281,6 +286,7 @@ __global__ void __launch_bounds__(128) k_mingru_chunk(PassTables t, GruBranch b,
 template <typename OT>
 __global__ void __launch_bounds__(128) k_mingru_chunk_out(PassTables t, GruBranch b, const float* __restrict__ P, int ldp, int S, int C,
                                                           float* __restrict__ AB, const float* __restrict__ state, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     int seg, ck, first;
     if (!gru_find_chunk(t, S, C, blockIdx.x, seg, ck, first)) return;
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
@@ -310,6 +316,7 @@ __global__ void __launch_bounds__(128) k_mingru_chunk_out(PassTables t, GruBranc
     if ((ck + 1) * C >= len) AB[((size_t)blockIdx.x * 2 + 1) * b.width + c] = Sx;
 }
 __global__ void __launch_bounds__(128) k_mingru_store(PassTables t, GruBranch b, int S, int C, const float* __restrict__ AB, float* __restrict__ state) {
+    pdl_trigger_and_wait();
     const int seg = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
     if (c >= b.width) return;
     int last = -1;
@@ -357,6 +364,7 @@ __host__ __device__ __forceinline__ int sa_maps(const SoftAttn& b) { return b.ma
 // q (and k): per-head norm, rotary positions; q in place (fp32), k and v appended to the slot's cache.
 template <typename OT>
 __global__ void __launch_bounds__(128) k_sattn_prep(PassTables t, SoftAttn b, float* __restrict__ P, int ldp, OT* __restrict__ kc, OT* __restrict__ vc) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int slot = t.seg_slot[t.row_seg[r]], pos = t.row_pos[r];
     float* p = P + (size_t)r * ldp;
@@ -405,6 +413,7 @@ __global__ void __launch_bounds__(128) k_sattn_prep(PassTables t, SoftAttn b, fl
 template <typename OT>
 __global__ void __launch_bounds__(128) k_pool_update(PassTables t, SoftAttn b, const OT* __restrict__ kc, const OT* __restrict__ vc,
                                                      float* __restrict__ pk, float* __restrict__ pv) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x;
     const int slot = t.seg_slot[t.row_seg[r]], pos = t.row_pos[r];
     if ((pos + 1) % b.pool != 0) return;
@@ -467,6 +476,7 @@ __device__ __forceinline__ void sattn_sweep(const PassTables& t, const SoftAttn&
     const bool kvec = b.dim % 8 == 0 && kld % 8 == 0, pooled = b.keep <= 0;
     const float slope = b.slope ? b.slope[h / M] : 0.0f;
     const int pos = t.row_pos[r];
+    const int kg = nb == 0 && blockDim.x == 128 ? (b.vdim <= 32 ? 4 : b.vdim <= 64 ? 2 : 1) : 1;
     __syncthreads();
     for (int n0 = n_lo; n0 < n_hi; n0 += blockDim.x) {
         const int n = n0 + threadIdx.x;
@@ -483,6 +493,23 @@ __device__ __forceinline__ void sattn_sweep(const PassTables& t, const SoftAttn&
         l = l * corr + block_sum(pw, red);               // (its barriers also publish swt)
         m = mn;
         const int nj = min((int)blockDim.x, n_hi - n0);
+        if (kg > 1 || nb == 0) {                             // plain tokens: loads eight keys ahead of the sums; narrow heads: kg thread groups take every kg-th key
+            const int cw = blockDim.x / kg, grp = threadIdx.x / cw;
+#pragma unroll
+            for (int cc = 0; cc < 4; cc++) {
+                const int c = threadIdx.x % cw + cc * cw;
+                if (c < b.vdim) {
+                    float a = acc[cc] * corr;
+                    const OT* vr = vbase + (size_t)(lo + n0) * vld + c;
+#pragma unroll 8
+                    for (int jj = grp; jj < nj; jj += kg) a = fmaf(swt[jj], ldf<OT>(vr + (size_t)jj * vld), a);
+                    acc[cc] = a;
+                }
+                if (kg > 1) break;
+            }
+            __syncthreads();
+            continue;
+        }
 #pragma unroll
         for (int cc = 0; cc < 4; cc++) {
             const int c = threadIdx.x + cc * blockDim.x;
@@ -497,6 +524,13 @@ __device__ __forceinline__ void sattn_sweep(const PassTables& t, const SoftAttn&
             }
         }
         __syncthreads();
+    }
+    if (kg > 1) {                                            // the groups' sums meet in the first group's threads
+        const int cw = blockDim.x / kg;
+        swt[threadIdx.x] = acc[0];
+        __syncthreads();
+        if ((int)threadIdx.x < cw)
+            for (int q = 1; q < kg; q++) acc[0] += swt[q * cw + threadIdx.x];
     }
 }
 template <typename OT>
@@ -519,6 +553,7 @@ __device__ __forceinline__ void sattn_store(const SoftAttn& b, const float* __re
 template <typename OT, typename OUT = OT>
 __global__ void __launch_bounds__(128) k_sattn(PassTables t, SoftAttn b, const float* __restrict__ P, int ldp, const OT* __restrict__ kc, const OT* __restrict__ vc,
                                                const float* __restrict__ pk, const float* __restrict__ pv, OUT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     extern __shared__ float sm[];
     const int r = blockIdx.x, h = blockIdx.y, pos = t.row_pos[r];
     int lo, nb;
@@ -536,6 +571,7 @@ template <typename OT>
 __global__ void __launch_bounds__(128) k_sattn_split(PassTables t, SoftAttn b, const float* __restrict__ P, int ldp, const OT* __restrict__ kc,
                                                      const OT* __restrict__ vc, const float* __restrict__ pk, const float* __restrict__ pv,
                                                      float* __restrict__ part, int R) {
+    pdl_trigger_and_wait();
     extern __shared__ float sm[];
     const int r = blockIdx.x, h = blockIdx.y, pos = t.row_pos[r];
     int lo, nb;
@@ -557,6 +593,7 @@ __global__ void __launch_bounds__(128) k_sattn_split(PassTables t, SoftAttn b, c
 template <typename OT>
 __global__ void __launch_bounds__(128) k_sattn_join(SoftAttn b, const float* __restrict__ P, int ldp, const float* __restrict__ part, int R, int splits,
                                                     OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     // splits <= 32: one warp fetches every split's maximum and denominator at once and turns them into the splits' weights; the value sums
     // are then folded in order without waiting on a load per split
     __shared__ float sw[32];
@@ -602,6 +639,7 @@ __global__ void __launch_bounds__(128) k_sattn_join(SoftAttn b, const float* __r
 template <typename OT>
 __global__ void __launch_bounds__(256) k_polynorm(const float* __restrict__ G, int ldg, int ff, float eps, const float* __restrict__ coef,
                                                   OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     __shared__ float red[3][9];
     const int r = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float* z = G + (size_t)r * ldg;
@@ -673,6 +711,7 @@ template <typename OT>
 __global__ void __launch_bounds__(256) k_moe_up_rows(const OT* __restrict__ X, int ldx, int K, const bf16* __restrict__ w_up, int ldw, int ff, int kfp,
                                                      int n_experts, int top, const int* __restrict__ sel_idx, const float* __restrict__ sel_w,
                                                      OT* __restrict__ act) {
+    pdl_trigger_and_wait();
     const int pair = blockIdx.x, r = pair / top, e = sel_idx[pair];
     if (e >= n_experts) return;
     const float wt = sel_w[pair];
@@ -688,6 +727,7 @@ __global__ void __launch_bounds__(256) k_moe_up_rows(const OT* __restrict__ X, i
 template <typename OT>
 __global__ void __launch_bounds__(256) k_moe_down_rows(const OT* __restrict__ act, int kfp, const bf16* __restrict__ w_down, int width, int n_experts, int top,
                                                        const int* __restrict__ sel_idx, float* __restrict__ Y, int ldy) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int c = blockIdx.y * nw + warp; c < width; c += gridDim.y * nw) {
         float y = 0.0f;

@@ -23,6 +23,7 @@ template <int DP, int VP>
 __global__ void __launch_bounds__(128) k_sattn_mma(PassTables t, SoftAttn b, int S, const float* __restrict__ P, int ldp, const bf16* __restrict__ kc,
                                                    const bf16* __restrict__ vc, const float* __restrict__ pk, const float* __restrict__ pv,
                                                    bf16* __restrict__ out, int ld_out, float* __restrict__ out_f, int ld_f) {
+    pdl_trigger_and_wait();
     constexpr int LQ = DP + 8, LV = VP + 8;
     extern __shared__ __align__(16) unsigned char sa_raw[];
     bf16* sq = reinterpret_cast<bf16*>(sa_raw);          // [64][LQ]
@@ -228,6 +229,7 @@ __global__ void __launch_bounds__(128) k_sattn_mma(PassTables t, SoftAttn b, int
 // (dst; -1 for an identity expert) and every M tile its expert (tile_e; -1 beyond the last group).  Shared memory: 2 n_experts ints.
 __global__ void __launch_bounds__(1024) k_moe_group(const int* __restrict__ sel_idx, int n_pairs, int n_experts, int* __restrict__ dst,
                                                     int* __restrict__ tile_e, int n_tiles) {
+    pdl_trigger_and_wait();
     extern __shared__ int sg[];
     int* cnt = sg;                  // [n_experts] pairs per expert, then the running fill of the group
     int* start = sg + n_experts;    // [n_experts] first row of the group
@@ -255,6 +257,7 @@ __global__ void __launch_bounds__(1024) k_moe_group(const int* __restrict__ sel_
 // Xg[dst[pair]] = X[pair / top] (bf16 rows of ld elements, 16-byte pieces); rw[dst[pair]] = the pair's weight
 __global__ void __launch_bounds__(128) k_moe_gather(const bf16* __restrict__ X, int ld, int top, const int* __restrict__ dst, const float* __restrict__ sel_w,
                                                     bf16* __restrict__ Xg, float* __restrict__ rw) {
+    pdl_trigger_and_wait();
     const int pair = blockIdx.x, d = dst[pair];
     if (d < 0) return;
     const uint4* src = reinterpret_cast<const uint4*>(X + (size_t)(pair / top) * ld);

@@ -68,6 +68,7 @@ __device__ __forceinline__ void delta_gates(const RecBranch& b, const float* __r
 template <int KIND>
 __global__ void __launch_bounds__(1024) k_rec_gates(PassTables t, RecBranch b, const float* __restrict__ P, int ldp, int C, float* __restrict__ mstate, float4* __restrict__ G,
                                                    float2* __restrict__ Bp) {
+    pdl_trigger_and_wait();
     __shared__ float sF[32], sM[32];
     __shared__ double sB[32];
     const int s = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(1024) k_rec_gates(PassTables t, RecBranch b, c
 
 // unit length: every head of q and k (X columns q_off.. and k_off.., kv_heads each) divided by sqrt(sum of squares + 1e-6), q times qscale; in place
 __global__ void __launch_bounds__(128) k_rec_unit(RecBranch b, float* __restrict__ X, int ldx) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int u = blockIdx.y * nw + wid; u < 2 * b.kv_heads; u += gridDim.y * nw) {
         const bool is_q = u < b.kv_heads;
@@ -140,6 +142,7 @@ __global__ void __launch_bounds__(128) k_rec_unit(RecBranch b, float* __restrict
 template <int KIND, int RPT, bool ONE>
 __global__ void __launch_bounds__(256) k_rec_walk(PassTables t, RecBranch b, const float* __restrict__ X, int ldx, const float* __restrict__ P, int ldp, const float4* __restrict__ G,
                                                   const float* __restrict__ mstate, float* __restrict__ state, float* __restrict__ O) {
+    pdl_trigger_and_wait();
     constexpr int DP = RPT * 8, NPF = (DP + 255) / 256;
     __shared__ __align__(16) float sq[2][DP], sk[2][DP];
     __shared__ float part[2][2][8][32], skq[2][3][8];
@@ -240,6 +243,7 @@ __global__ void __launch_bounds__(256) k_rec_walk(PassTables t, RecBranch b, con
 template <typename OT, int KIND>
 __global__ void __launch_bounds__(128) k_rec_post(PassTables t, RecBranch b, const float* __restrict__ O, const float4* __restrict__ G, float* __restrict__ mstate,
                                                   const float* __restrict__ P, int ldp, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int h = blockIdx.y * nw + wid; h < b.heads; h += gridDim.y * nw) {
         const float* o = O + (size_t)r * (b.heads * b.vx) + h * b.vx;
@@ -281,6 +285,7 @@ __global__ void __launch_bounds__(128) k_rec_post(PassTables t, RecBranch b, con
 template <int KIND>
 __global__ void __launch_bounds__(256) k_rec_prep(RecBranch b, const float* __restrict__ X, int ldx, bf16* __restrict__ QP, bf16* __restrict__ KP, size_t ps_qk,
                                                   bf16* __restrict__ VPn, size_t ps_v) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const float* x = X + (size_t)r * ldx;
     const int units = 2 * b.kv_heads + b.heads;
@@ -339,6 +344,7 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 template <int C>
 __global__ void __launch_bounds__(256, 2) k_delta_wy(PassTables t, RecBranch b, int S, const bf16* __restrict__ KP, size_t ps_qk, const bf16* __restrict__ VPn, size_t ps_v,
                                                      const float4* __restrict__ G, const float2* __restrict__ Bp, float* __restrict__ X, int ldx, bf16* __restrict__ WP, size_t ps_w) {
+    pdl_trigger_and_wait();
     extern __shared__ __align__(16) unsigned char rc_raw[];
     __shared__ float sbeta[C], sbeb[C], sbh[C], sbl[C];
     constexpr int LA = C + 4, NB = C / 16;
@@ -495,6 +501,7 @@ template <int KIND, int C, int MT>
 __global__ void __launch_bounds__(256) k_rec_scan(PassTables t, RecBranch b, const bf16* __restrict__ KP, size_t ps_qk, const bf16* __restrict__ WP, size_t ps_w,
                                                   const float4* __restrict__ G, const float2* __restrict__ Bp, const float* __restrict__ X, int ldx, bf16* __restrict__ UP, size_t ps_v,
                                                   bf16* __restrict__ SP, float* __restrict__ state) {
+    pdl_trigger_and_wait();
     extern __shared__ __align__(16) unsigned char rc_raw[];
     constexpr int LS = REC_VS + 8;
     const int LK = b.dp + 8;
@@ -675,6 +682,7 @@ template <int VP, int C>
 __global__ void __launch_bounds__(2 * C) k_rec_out(PassTables t, RecBranch b, int kind, int S, const bf16* __restrict__ QP, const bf16* __restrict__ KP, size_t ps_qk,
                                                    const bf16* __restrict__ UP, size_t ps_v, const bf16* __restrict__ SP, const float4* __restrict__ G, const float2* __restrict__ Bp,
                                                    float* __restrict__ O) {
+    pdl_trigger_and_wait();
     extern __shared__ __align__(16) unsigned char rc_raw[];
     constexpr int LQ = 64 + 8, LV = VP + 8;
     bf16* sq = reinterpret_cast<bf16*>(rc_raw);              // [2][C][LQ]
@@ -806,6 +814,7 @@ constexpr int SSM_SERVE = 384;
 template <typename OT, int LANES, int KS, int TILE>
 __global__ void __launch_bounds__(128 + SSM_SERVE, 1) k_ssm_scan(PassTables t, SsmBranch b, const float* __restrict__ XC, const float* __restrict__ DT, const float* __restrict__ BC, int ld_bc,
                                                   const float* __restrict__ P, int ldp, float* __restrict__ state, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     constexpr int NCH = 128 / LANES, NSP = LANES * KS, NE = (TILE * NCH + SSM_SERVE - 1) / SSM_SERVE;      // NE: (row, channel) pairs of a tile per serving thread
     __shared__ __align__(16) float sB[2][TILE][NSP], sC[2][TILE][NSP];
     __shared__ float2 sdx[2][TILE][NCH];                  // {dt, dt x}
@@ -963,6 +972,7 @@ __global__ void __launch_bounds__(128 + SSM_SERVE, 1) k_ssm_scan(PassTables t, S
 // columns [0, n) of an fp32 block as a product operand, zero-padded to ld_out
 template <typename OT>
 __global__ void k_cols_operand(const float* __restrict__ A, int lda, int n, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x;
     for (int c = threadIdx.x; c < ld_out; c += blockDim.x) out[(size_t)r * ld_out + c] = cvt<OT>(c < n ? A[(size_t)r * lda + c] : 0.0f);
 }

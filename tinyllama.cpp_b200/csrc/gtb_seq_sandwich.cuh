@@ -59,6 +59,7 @@ __device__ __forceinline__ void sw_stats(const float (&v)[4 * N4], int width, in
 template <typename OT>
 __global__ void __launch_bounds__(256) k_norm_rows(const float* __restrict__ x, int width, NormArgs nrm, const int* __restrict__ rows, OT* __restrict__ out, int ld_out,
                                                    float out_scale) {
+    pdl_trigger_and_wait();
     __shared__ float red[33];
     const int o = blockIdx.x, r = rows ? rows[o] : o, center = nrm.kind == SW_NORM_LAYER;
     const float* xr = x + (size_t)r * width;
@@ -129,6 +130,7 @@ __device__ __forceinline__ void route_grouped_row(const float* __restrict__ z, i
 // rows of router logits Z -> choices; sel_idx / sel_w [rows][top + n_always].  Shared memory: 2 n_exp + n_groups floats.
 __global__ void __launch_bounds__(32) k_moe_route_grouped(const float* __restrict__ Z, int ldz, int n_exp, int n_groups, int keep, int top, float scale,
                                                           int n_always, int* __restrict__ sel_idx, float* __restrict__ sel_w) {
+    pdl_trigger_and_wait();
     extern __shared__ float rsm[];
     const int r = blockIdx.x, tt = top + n_always;
     route_grouped_row(Z + (size_t)r * ldz, n_exp, n_groups, keep, top, scale, n_always, sel_idx + (size_t)r * tt, sel_w + (size_t)r * tt, rsm, rsm + n_exp,
@@ -163,6 +165,7 @@ __device__ __forceinline__ void route_top_softmax_row(const float* __restrict__ 
     if (lane + 32 < top) sel_w[lane + 32] = e1 * inv;
 }
 __global__ void __launch_bounds__(32) k_moe_route_softmax(const float* __restrict__ Z, int ldz, int n_exp, int top, int* __restrict__ sel_idx, float* __restrict__ sel_w) {
+    pdl_trigger_and_wait();
     extern __shared__ float rsm[];
     const int r = blockIdx.x;
     route_top_softmax_row(Z + (size_t)r * ldz, n_exp, top, sel_idx + (size_t)r * top, sel_w + (size_t)r * top, rsm, threadIdx.x);
@@ -211,6 +214,7 @@ __device__ __forceinline__ void sandwich_route(const GroupRouteNext& rn, float* 
 template <typename OT>
 __global__ void __launch_bounds__(256) k_embed_norm(PassTables t, const bf16* __restrict__ embed, int width, float scale, NormArgs nrm, float* __restrict__ x,
                                                     OT* __restrict__ op, int ld_op) {
+    pdl_trigger_and_wait();
     __shared__ float red[33];
     const int r = blockIdx.x, center = nrm.kind == SW_NORM_LAYER;
     const bf16* e = embed + (size_t)t.tok[r] * width;
@@ -237,6 +241,7 @@ template <typename OT, int SW_KEEP, bool JOIN = false>
 __global__ void __launch_bounds__(256, JOIN ? (SW_KEEP == 4 ? 2 : 4) : SW_KEEP == 4 ? 4 : SW_KEEP == 2 ? 6 : 8) k_sandwich_add(const float* __restrict__ Y, const float* __restrict__ Y2, const float* __restrict__ Yg,
                                                       const int* __restrict__ pair_dst, int top, int width, NormArgs post, float* __restrict__ x,
                                                       NormArgs next, OT* __restrict__ op, int ld_op, GroupRouteNext rn, JoinArgs jn) {
+    pdl_trigger_and_wait();
     __shared__ float red[JOIN ? 192 : 128];           // four reductions (two more to join branches), each with 32 floats of its own (the walking path uses the first 33)
     __shared__ int sdst[PN_MAX_TOP];
     extern __shared__ float srt[];
@@ -356,6 +361,7 @@ __global__ void __launch_bounds__(256, JOIN ? (SW_KEEP == 4 ? 2 : 4) : SW_KEEP =
 
 // sc[r][0] = 1 / sqrt(mean(q_r^2) + eps) over the nq entries of row r's query projection, sc[r][1] the same for its nk key entries (nk may be 0)
 __global__ void __launch_bounds__(256) k_proj_rms(const float* __restrict__ P, int ldp, int q_off, int nq, int k_off, int nk, float eps, float* __restrict__ sc) {
+    pdl_trigger_and_wait();
     __shared__ float red[33];
     const int r = blockIdx.x;
     const float* p = P + (size_t)r * ldp;
@@ -381,6 +387,7 @@ struct DiffArgs {
 // o / sqrt(mean(o^2) + eps) * (1 - diff), gate, weight -> operand.  A warp per (row, head).
 template <typename OT>
 __global__ void __launch_bounds__(128) k_diff_combine(DiffArgs b, const float* __restrict__ A, const float* __restrict__ P, int ldp, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float d1 = 0.0f, d2 = 0.0f;
     for (int i = lane; i < b.dim; i += 32) { d1 = fmaf(b.lq1[i], b.lk1[i], d1); d2 = fmaf(b.lq2[i], b.lk2[i], d2); }
@@ -400,6 +407,7 @@ __global__ void __launch_bounds__(128) k_diff_combine(DiffArgs b, const float* _
 // ------------------------------------------------------------------------------------------------ retention: activation, joint norm
 // q, k, v <- silu(.) in place: columns [c0, c0 + n) of the projection buffer (q | k | v are neighbours)
 __global__ void k_silu_cols(float* __restrict__ P, int ldp, int c0, int n, int R) {
+    pdl_trigger_and_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)R * n) return;
     float* p = P + (i / n) * ldp + c0 + (i % n);
@@ -410,6 +418,7 @@ __global__ void k_silu_cols(float* __restrict__ P, int ldp, int c0, int n, int R
 template <typename OT>
 __global__ void __launch_bounds__(256) k_ret_post_all(RetBranch b, const float* __restrict__ w, const float* __restrict__ O, const float* __restrict__ P, int ldp,
                                                       OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     __shared__ float red[33];
     const int r = blockIdx.x, n = b.heads * b.vdim;
     const float* o = O + (size_t)r * n;
@@ -449,6 +458,7 @@ template <typename T> __device__ __forceinline__ void cv_store(T* p, const float
 template <typename OT, int V, int TAPS>
 __global__ void __launch_bounds__(128) k_qk_conv(PassTables t, ConvArgs b, const float* __restrict__ P, int ldp, int R, int rows_per, float* __restrict__ tail,
                                                  float* __restrict__ Q, OT* __restrict__ kc, OT* __restrict__ vc, int every_one) {
+    pdl_trigger_and_wait();
     const int nc = b.nq + b.nk, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
     if (c >= nc + b.nv) return;
     const int r0 = blockIdx.x * rows_per, r1 = min(R, r0 + rows_per);
@@ -532,6 +542,7 @@ __global__ void __launch_bounds__(128) k_qk_conv(PassTables t, ConvArgs b, const
 // act = gelu(G) -> operand [R][ld_out], zero-padded (grid: rows x column groups; few rows spread their columns over many CTAs)
 template <typename OT>
 __global__ void k_gelu_rows(const float* __restrict__ G, int ff, OT* __restrict__ out, int ld_out) {
+    pdl_trigger_and_wait();
     const int r = blockIdx.x;
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < ld_out; c += gridDim.y * blockDim.x)
         out[(size_t)r * ld_out + c] = cvt<OT>(c < ff ? gelu_erf(G[(size_t)r * ff + c]) : 0.0f);

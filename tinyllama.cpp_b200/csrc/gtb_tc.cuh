@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 namespace gtb {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -100,6 +102,29 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 __device__ __forceinline__ void pdl_trigger_and_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Launch with programmatic dependent launch (and an optional cluster of `cluster` CTAs along x): the kernel may start while its predecessor
+// drains, so it MUST call pdl_wait (or pdl_trigger_and_wait) before it touches anything that earlier kernels write or still read.  A kernel that
+// allocates TMEM triggers its successor only behind the allocation: an early successor could otherwise hold the columns that it waits for.
+template <typename... P, typename... A>
+inline void pdl_launch_cluster(int cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = grid; lc.blockDim = block; lc.dynamicSmemBytes = smem; lc.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = cluster > 0 ? 2 : 1;
+    (void)cudaLaunchKernelEx(&lc, kernel, std::forward<A>(args)...);      // (the caller's GTB_LAUNCHED looks at the error)
+}
+template <typename... P, typename... A>
+inline void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    pdl_launch_cluster(0, kernel, grid, block, smem, st, std::forward<A>(args)...);
 }
 
 // shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: rows are 128 B apart, 8-row groups 1024 B
