@@ -205,7 +205,10 @@ struct gtb_seq_model {
     int *d_row_pos = nullptr, *d_row_prev = nullptr, *d_hist = nullptr;
     SlotState* d_slots = nullptr;
     std::vector<int> host_pos;
-    std::vector<char> host_stopped_unknown;
+    int *d_step = nullptr, *d_dec = nullptr;     // device-driven decode: number of the step in its call, sampled tokens [step][row]
+    StateArray* d_state = nullptr;               // every array with a share per slot (what a reset clears)
+    int n_state = 0;
+    char* h_back = nullptr;                      // pinned: [status word | SlotState of every slot], read back with a call's results
     int last_nseg = 0;                           // rows of `logits` that hold segment-last rows (greedy / decode)
     bool use_tensor = true;
     int tensor_min_rows = 64;                    // rows from which routed experts run as grouped products and the scan's step sizes from bf16 operands
@@ -1491,7 +1494,7 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
             GTB_LAUNCHED();
         }
     }
-    pdl_launch(k_commit, (S + 127) / 128, 128, 0, st, t, S);
+    pdl_launch(k_commit, (S + 127) / 128, 128, 0, st, t, S, from_pending ? m->d_step : nullptr);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -2253,7 +2256,28 @@ int gtb_seq_create(gtb_seq_t* out, const gtb_seq_config* cfg, const gtb_seq_laye
     GTB_CUDA(cudaHostAlloc((void**)&m->h_tab, m->tab_cap * sizeof(int), cudaHostAllocDefault));
     TRY(dalloc_t(m, &m->d_row_pos, R));
     TRY(dalloc_t(m, &m->d_row_prev, R));
-    TRY(dalloc_t(m, &m->d_hist, (size_t)c.n_slots * 2));
+    TRY(dalloc_t(m, &m->d_hist, (size_t)c.n_slots));
+    TRY(dalloc_t(m, &m->d_step, 1));
+    TRY(dalloc_t(m, &m->d_dec, (size_t)c.n_slots * c.max_ctx));
+    GTB_CUDA(cudaHostAlloc((void**)&m->h_back, 16 + c.n_slots * sizeof(SlotState), cudaHostAllocDefault));
+    {
+        std::vector<StateArray> arrays;
+        for (const Run& r : m->runs) {
+            const LayerW& l = m->L[r.layer];
+            for (int bi = 0; bi < l.d.n_branches; bi++) {
+                if (r.state[bi]) arrays.push_back({r.state[bi], state_floats(l.br[bi].d)});
+                if (r.mstate[bi]) arrays.push_back({r.mstate[bi], (size_t)l.br[bi].d.heads});
+            }
+            if (r.ctail) arrays.push_back({r.ctail, (size_t)r.ctail_n});
+            if (r.tail) arrays.push_back({r.tail, (size_t)(c.taps - 1) * W});
+        }
+        m->n_state = (int)arrays.size();
+        TRY(dalloc_t(m, &m->d_state, arrays.size()));
+        if (!arrays.empty()) {
+            GTB_CUDA(cudaMemcpyAsync(m->d_state, arrays.data(), arrays.size() * sizeof(StateArray), cudaMemcpyHostToDevice, ctx().stream));
+            GTB_CUDA(cudaStreamSynchronize(ctx().stream));
+        }
+    }
     TRY(dalloc_t(m, &m->d_slots, c.n_slots));
     m->host_pos.assign(c.n_slots, 0);
     for (int s = 0; s < c.n_slots; s++) TRY(gtb_seq_slot_reset(m, s));
@@ -2270,6 +2294,7 @@ int gtb_seq_destroy(gtb_seq_t m) {
     cudaStreamSynchronize(ctx().stream);
     if (m->graph) cudaGraphExecDestroy(m->graph);
     if (m->gp) seq_gemm_destroy(m->gp);
+    if (m->h_back) cudaFreeHost(m->h_back);
     for (void* p : m->allocs) cudaFree(p);
     if (m->h_tab) cudaFreeHost(m->h_tab);
     delete m;
@@ -2325,24 +2350,8 @@ int gtb_seq_n_runs(gtb_seq_t m, int* n) { GTB_ARG(m && n); *n = (int)m->runs.siz
 int gtb_seq_slot_reset(gtb_seq_t m, int slot) {
     GTB_CHECK_INIT();
     GTB_ARG(m && slot >= 0 && slot < m->cfg.n_slots);
-    cudaStream_t st = ctx().stream;
-    const SlotState z{0, -1, 0, 0};
-    GTB_CUDA(cudaMemcpyAsync(m->d_slots + slot, &z, sizeof z, cudaMemcpyHostToDevice, st));
-    GTB_CUDA(cudaStreamSynchronize(st));                    // z is a local
-    for (Run& r : m->runs) {
-        const LayerW& l = m->L[r.layer];
-        for (int bi = 0; bi < l.d.n_branches; bi++)
-            if (r.state[bi]) {
-                const size_t sb = state_floats(l.br[bi].d) * sizeof(float);
-                GTB_CUDA(cudaMemsetAsync((char*)r.state[bi] + sb * slot, 0, sb, st));
-                if (r.mstate[bi]) GTB_CUDA(cudaMemsetAsync(r.mstate[bi] + (size_t)l.br[bi].d.heads * slot, 0, l.br[bi].d.heads * sizeof(float), st));
-            }
-        if (r.ctail) GTB_CUDA(cudaMemsetAsync(r.ctail + (size_t)r.ctail_n * slot, 0, r.ctail_n * sizeof(float), st));
-        if (r.tail) {
-            const size_t tb = (size_t)(m->cfg.taps - 1) * m->cfg.width * sizeof(float);
-            GTB_CUDA(cudaMemsetAsync((char*)r.tail + tb * slot, 0, tb, st));
-        }
-    }
+    pdl_launch(k_slot_reset, dim3(m->n_state + 1, 32), 256, 0, ctx().stream, m->d_state, m->n_state, m->d_slots, slot);
+    GTB_LAUNCHED();
     m->host_pos[slot] = 0;
     return GTB_OK;
 }
@@ -2415,6 +2424,7 @@ static int step_impl(gtb_seq_t m, int n_seg, const int32_t* seg_slot, const int3
         const PassTables t = tables(m, S, R);
         const int* d_want = m->d_tab + 3 * S + 2 * R;
         int rc;
+        int* h_status = reinterpret_cast<int*>(m->h_back);       // comes back with the pass's results, behind one wait
         // greedy passes: logits rows are ordered like greedy_segs; the argmax kernel needs a segment per logits row, so it runs on
         // a table of its own below
         if (c.mode == GTB_SEQ_F32) rc = run_pass<float>(m, t, R, S, false, nw, d_want, pl.data(), ps.data());
@@ -2427,17 +2437,20 @@ static int step_impl(gtb_seq_t m, int n_seg, const int32_t* seg_slot, const int3
             GTB_CUDA(cudaMemcpyAsync(m->d_tab + n_ints, m->h_tab + n_ints, nw * sizeof(int), cudaMemcpyHostToDevice, st));
             PassTables ta = t;
             ta.seg_slot = m->d_tab + n_ints;
-            pdl_launch(k_argmax_rows, nw, 1024, 0, st, m->logits, c.vocab, ta, -1, m->d_hist, 1, 0);
+            pdl_launch(k_argmax_rows, nw, 1024, 0, st, m->logits, c.vocab, ta, -1, m->d_hist, nullptr);
             GTB_LAUNCHED();
             std::vector<int> got(nw);
             GTB_CUDA(cudaMemcpyAsync(got.data(), m->d_hist, nw * sizeof(int), cudaMemcpyDeviceToHost, st));
+            if (m->gp && (rc = seq_gemm_status_async(m->gp, h_status))) return rc;
             GTB_CUDA(cudaStreamSynchronize(st));
             for (int i = 0; i < nw; i++) h_next[pseg_of[greedy_segs[i]]] = got[i];
             m->last_nseg = nw;
         } else if (nw) {
+            if (m->gp && (rc = seq_gemm_status_async(m->gp, h_status))) return rc;
             GTB_CUDA(cudaMemcpyAsync(h_logits + (size_t)(wi - nw) * c.vocab, m->logits, (size_t)nw * c.vocab * sizeof(float), cudaMemcpyDeviceToHost, st));
             GTB_CUDA(cudaStreamSynchronize(st));
         } else {
+            if (m->gp && (rc = seq_gemm_status_async(m->gp, h_status))) return rc;
             GTB_CUDA(cudaStreamSynchronize(st));       // the pinned table buffer is reused by the next pass
         }
         for (int k = 0; k < S; k++) m->host_pos[ps[k]] += pl[k];
@@ -2445,12 +2458,8 @@ static int step_impl(gtb_seq_t m, int n_seg, const int32_t* seg_slot, const int3
         seg = s; off = o;
     }
     (void)next;
-    if (m->gp) {
-        int bad = 0;
-        int rc = seq_gemm_status(m->gp, &bad);
-        if (rc) return rc;
-        if (bad) return gtb::fail(GTB_ERR_STATE, "a tensor-core product gave up on a pipeline wait; results of this step are not valid");
-    }
+    if (m->gp && *reinterpret_cast<const int*>(m->h_back))
+        return gtb::fail(GTB_ERR_STATE, "a tensor-core product gave up on a pipeline wait; results of this step are not valid");
     return GTB_OK;
 }
 
@@ -2488,12 +2497,11 @@ int gtb_seq_decode(gtb_seq_t m, int n, const int32_t* slots, int n_steps, int eo
     GTB_CUDA(cudaMemcpyAsync(m->d_tab, m->h_tab, 6 * n * sizeof(int), cudaMemcpyHostToDevice, st));
     const PassTables t = tables(m, n, n);
     const int* d_want = m->d_tab + 5 * n;
-    int* d_out = nullptr;
-    GTB_CUDA(cudaMalloc((void**)&d_out, (size_t)n * n_steps * sizeof(int)));
+    GTB_CUDA(cudaMemsetAsync(m->d_step, 0xff, sizeof(int), st));        // -1: the first step's commit makes it 0
     auto one = [&]() -> int {
         int rc = c.mode == GTB_SEQ_F32 ? run_pass<float>(m, t, n, n, true, n, d_want) : run_pass<bf16>(m, t, n, n, true, n, d_want);
         if (rc) return rc;
-        pdl_launch(k_argmax_rows, n, 1024, 0, st, m->logits, c.vocab, t, eos_id, m->d_hist, 1, 0);
+        pdl_launch(k_argmax_rows, n, 1024, 0, st, m->logits, c.vocab, t, eos_id, m->d_dec, m->d_step);
         GTB_LAUNCHED();
         return GTB_OK;
     };
@@ -2507,11 +2515,11 @@ int gtb_seq_decode(gtb_seq_t m, int n, const int32_t* slots, int n_steps, int eo
             rc = one();
             cudaError_t ce = cudaStreamEndCapture(st, &g);
             ctx().launches = l0;
-            if (rc) { if (g) cudaGraphDestroy(g); cudaFree(d_out); return rc; }
-            if (ce != cudaSuccess) { cudaFree(d_out); return gtb::fail(GTB_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ce)); }
+            if (rc) { if (g) cudaGraphDestroy(g); return rc; }
+            if (ce != cudaSuccess) return gtb::fail(GTB_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ce));
             ce = cudaGraphInstantiate(&m->graph, g, 0);
             cudaGraphDestroy(g);
-            if (ce != cudaSuccess) { cudaFree(d_out); return gtb::fail(GTB_ERR_CUDA, "graph instantiation failed: %s", cudaGetErrorString(ce)); }
+            if (ce != cudaSuccess) return gtb::fail(GTB_ERR_CUDA, "graph instantiation failed: %s", cudaGetErrorString(ce));
             m->graph_slots.assign(slots, slots + n);
             m->graph_eos = eos_id;
         }
@@ -2524,20 +2532,22 @@ int gtb_seq_decode(gtb_seq_t m, int n, const int32_t* slots, int n_steps, int eo
         } else {
             rc = one();
         }
-        if (rc == GTB_OK) {
-            cudaError_t ce = cudaMemcpy2DAsync(d_out + k, (size_t)n_steps * sizeof(int), m->d_hist, sizeof(int), sizeof(int), n, cudaMemcpyDeviceToDevice, st);
-            if (ce != cudaSuccess) rc = gtb::fail(GTB_ERR_CUDA, "copy failed: %s", cudaGetErrorString(ce));
-        }
     }
-    if (rc == GTB_OK) {
-        cudaError_t ce = cudaMemcpyAsync(h_out, d_out, (size_t)n * n_steps * sizeof(int), cudaMemcpyDeviceToHost, st);
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-        if (ce != cudaSuccess) rc = gtb::fail(GTB_ERR_CUDA, "copy failed: %s", cudaGetErrorString(ce));
-    }
-    cudaFree(d_out);
     if (rc) return rc;
+    // tokens, slot positions and the status word behind one wait
+    std::vector<int> toks((size_t)n * n_steps);
+    int* h_status = reinterpret_cast<int*>(m->h_back);
+    SlotState* h_slots = reinterpret_cast<SlotState*>(m->h_back + 16);
+    *h_status = 0;
+    GTB_CUDA(cudaMemcpyAsync(h_slots, m->d_slots, c.n_slots * sizeof(SlotState), cudaMemcpyDeviceToHost, st));
+    if (m->gp && (rc = seq_gemm_status_async(m->gp, h_status))) return rc;
+    GTB_CUDA(cudaMemcpyAsync(toks.data(), m->d_dec, toks.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+    GTB_CUDA(cudaStreamSynchronize(st));
+    for (int k = 0; k < n_steps; k++)
+        for (int i = 0; i < n; i++) h_out[(size_t)i * n_steps + k] = toks[(size_t)k * n + i];
+    for (int i = 0; i < n; i++) m->host_pos[slots[i]] = h_slots[slots[i]].pos;
+    if (*h_status) return gtb::fail(GTB_ERR_STATE, "a tensor-core product gave up on a pipeline wait; results of these steps are not valid");
     m->last_nseg = n;
-    for (int i = 0; i < n; i++) { int pos; gtb_seq_slot_position(m, slots[i], &pos); }
     return GTB_OK;
 }
 

@@ -507,8 +507,13 @@ void seq_gemm_destroy(SeqGemmPlan* p) {
     delete p;
 }
 
-int seq_gemm_status(SeqGemmPlan* p, int* status) {
+int seq_gemm_status_async(SeqGemmPlan* p, int* status) {
     GTB_CUDA(cudaMemcpyAsync(status, p->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx().stream));
+    return GTB_OK;
+}
+int seq_gemm_status(SeqGemmPlan* p, int* status) {
+    int rc = seq_gemm_status_async(p, status);
+    if (rc) return rc;
     GTB_CUDA(cudaStreamSynchronize(ctx().stream));
     return GTB_OK;
 }

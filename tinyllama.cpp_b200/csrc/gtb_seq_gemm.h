@@ -34,6 +34,8 @@ int seq_gemm_bf16_grouped(SeqGemmPlan* p, const void* A, int lda, const void* W,
                           float* C, int ldc, void* act, int ld_act, const float* row_w);
 // 1 if a kernel of this plan gave up on a wait since the plan was created (its results are then not valid)
 int seq_gemm_status(SeqGemmPlan* p, int* status);
+// the same without waiting for the copy (to pinned memory)
+int seq_gemm_status_async(SeqGemmPlan* p, int* status);
 
 }  // namespace seq
 }  // namespace gtb

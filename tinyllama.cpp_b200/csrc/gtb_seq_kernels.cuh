@@ -118,14 +118,28 @@ __global__ void k_plan(PassTables t, int R, int from_pending) {
     t.row_pos[r] = pos;
     t.row_prev[r] = (r > row0) ? (from_pending ? st.pending : t.tok[r - 1]) : (pos == 0 ? -1 : st.prev);
 }
-__global__ void k_commit(PassTables t, int S) {
+// step_no (device-driven decode steps): the number of the step in its call, read by k_argmax_rows
+__global__ void k_commit(PassTables t, int S, int* step_no) {
     pdl_trigger_and_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s == 0 && step_no) ++*step_no;
     if (s >= S) return;
     SlotState& st = t.slots[t.seg_slot[s]];
     if (st.stopped) return;
     st.pos += t.seg_len[s];
     st.prev = t.tok[t.seg_row0[s] + t.seg_len[s] - 1];
+}
+// an empty sequence: the slot's share of every state array to zero, position 0.  grid (arrays + 1, blocks per array)
+struct StateArray { float* base; size_t per_slot; };
+__global__ void __launch_bounds__(256) k_slot_reset(const StateArray* __restrict__ arrays, int n_arrays, SlotState* slots, int slot) {
+    pdl_trigger_and_wait();
+    if ((int)blockIdx.x == n_arrays) {
+        if (blockIdx.y == 0 && threadIdx.x == 0) slots[slot] = SlotState{0, -1, 0, 0};
+        return;
+    }
+    const StateArray a = arrays[blockIdx.x];
+    float* p = a.base + a.per_slot * slot;
+    for (size_t i = (size_t)blockIdx.y * blockDim.x + threadIdx.x; i < a.per_slot; i += (size_t)gridDim.y * blockDim.x) p[i] = 0.0f;
 }
 
 // ------------------------------------------------------------------------------------------------ embedding
@@ -713,9 +727,9 @@ __global__ void k_concat2(const float* __restrict__ x, const float* __restrict__
 
 // ------------------------------------------------------------------------------------------------ sampling
 // first maximum of each logits row (lowest index wins ties, like the greedy loop of the single-model engine); the token becomes the
-// slot's pending token and lands in hist[row][step]; a slot that samples eos_id stops.
+// slot's pending token and lands in out[step][row]; a slot that samples eos_id stops.
 __global__ void __launch_bounds__(1024) k_argmax_rows(const float* __restrict__ logits, int n, PassTables t, int eos_id, int* __restrict__ out,
-                                                       int out_ld, int out_col) {
+                                                       const int* __restrict__ step_no) {
     pdl_trigger_and_wait();
     __shared__ float sv[32];
     __shared__ int si[32];
@@ -759,7 +773,7 @@ __global__ void __launch_bounds__(1024) k_argmax_rows(const float* __restrict__ 
             if (st.stopped) arg = st.pending;
             st.pending = arg;
             if (eos_id >= 0 && arg == eos_id) st.stopped = 1;
-            out[(size_t)s * out_ld + out_col] = arg;
+            out[(step_no ? (size_t)*step_no * gridDim.x : 0) + s] = arg;
         }
     }
 }
