@@ -318,14 +318,28 @@ int product(gtb_seq_model* m, const void* A, int lda, const bf16* W, int ldw, fl
         if (rc != -1) return rc;
     }
     if (M <= 8) {
-        if (M <= 1) pdl_launch(k_gemv_rows<OT, 1, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
-        else if (M <= 2) pdl_launch(k_gemv_rows<OT, 2, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
-        else if (M <= 4) pdl_launch(k_gemv_rows<OT, 4, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
-        else pdl_launch(k_gemv_rows<OT, 8, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
+        if (M <= 1) pdl_launch(k_gemv_rows<OT, 1, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc, 0);
+        else if (M <= 2) pdl_launch(k_gemv_rows<OT, 2, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc, 0);
+        else if (M <= 4) pdl_launch(k_gemv_rows<OT, 4, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc, 0);
+        else pdl_launch(k_gemv_rows<OT, 8, 4>, (N + 3) / 4, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc, 0);
     } else {
         dim3 grid((N + SG_BN - 1) / SG_BN, (M + SG_BM - 1) / SG_BM);
         pdl_launch(k_gemm_simt<OT>, grid, 256, 0, st, a, lda, W, ldw, C, ldc, M, N, Kp, bias, acc);
     }
+    GTB_LAUNCHED();
+    return GTB_OK;
+}
+
+// Few rows (at most 8): the gated activation leaves the weight-streaming product (ACT 2: silu(gate) * up * row_w, 3: gelu_tanh(gate) * up); `pad` columns
+// behind the ff activations are written as zeros
+template <typename OT, int ACT>
+int gated_rows(const OT* a, int lda, const bf16* W, int ldw, OT* out, int ld_out, int R, int ff, int K, bool inter, const float* row_w, int pad) {
+    cudaStream_t st = ctx().stream;
+    const int grid = (ff + 1) / 2, il = inter ? 1 : 0;
+    if (R <= 1) pdl_launch(k_gemv_rows<OT, 1, 4, ACT, OT>, grid, 256, 0, st, a, lda, W, ldw, out, ld_out, R, 2 * ff, K, row_w, pad, il);
+    else if (R <= 2) pdl_launch(k_gemv_rows<OT, 2, 4, ACT, OT>, grid, 256, 0, st, a, lda, W, ldw, out, ld_out, R, 2 * ff, K, row_w, pad, il);
+    else if (R <= 4) pdl_launch(k_gemv_rows<OT, 4, 4, ACT, OT>, grid, 256, 0, st, a, lda, W, ldw, out, ld_out, R, 2 * ff, K, row_w, pad, il);
+    else pdl_launch(k_gemv_rows<OT, 8, 4, ACT, OT>, grid, 256, 0, st, a, lda, W, ldw, out, ld_out, R, 2 * ff, K, row_w, pad, il);
     GTB_LAUNCHED();
     return GTB_OK;
 }
@@ -1072,6 +1086,11 @@ int run_gated_experts(gtb_seq_model* m, int R, const LayerW& l, bool is_routed, 
             if (rc > 0) return rc;
             if (rc == 0) { ctx().launches++; act_done = true; }
         }
+        if (!act_done && R <= 8) {
+            rc = gated_rows<OT, 2>((const OT*)opA, wp, l.w_sh_gu, wp, (OT*)opC, l.sff_p, R, l.sff, wp, l.sh_inter, m->shw, l.sff_p - l.sff);
+            if (rc) return rc;
+            act_done = true;
+        }
         if (!act_done) {
             rc = product<OT>(m, opA, wp, l.w_sh_gu, wp, m->G, 2 * l.sff, R, 2 * l.sff, wp, nullptr, 0);
             if (rc) return rc;
@@ -1171,10 +1190,10 @@ int run_sandwich_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
         if (!act_done && R <= 8) {          // few rows: the activation leaves the weight-streaming product
             const OT* a = opA;
             const dim3 grid((l.ff + 3) / 4);
-            if (R <= 1) pdl_launch(k_gemv_rows<OT, 1, 4, true, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
-            else if (R <= 2) pdl_launch(k_gemv_rows<OT, 2, 4, true, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
-            else if (R <= 4) pdl_launch(k_gemv_rows<OT, 4, 4, true, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
-            else pdl_launch(k_gemv_rows<OT, 8, 4, true, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0);
+            if (R <= 1) pdl_launch(k_gemv_rows<OT, 1, 4, 1, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0, 0);
+            else if (R <= 2) pdl_launch(k_gemv_rows<OT, 2, 4, 1, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0, 0);
+            else if (R <= 4) pdl_launch(k_gemv_rows<OT, 4, 4, 1, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0, 0);
+            else pdl_launch(k_gemv_rows<OT, 8, 4, 1, OT>, grid, 256, 0, st, a, wp, l.w_up, wp, opC, l.kfp, R, l.ff, wp, nullptr, 0, 0);
             GTB_LAUNCHED();
             act_done = true;
         }
@@ -1196,6 +1215,11 @@ int run_sandwich_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
             rc = seq_gemm_bf16_gated(m->gp, opA, wp, l.w_gu, wp, opC, l.kfp, 0, R, 2 * l.ff, wp, 1, nullptr);
             if (rc > 0) return rc;
             if (rc == 0) { ctx().launches++; act_done = true; }
+        }
+        if (!act_done && R <= 8) {
+            rc = gated_rows<OT, 2>(opA, wp, l.w_gu, wp, opC, l.kfp, R, l.ff, wp, l.gu_inter, nullptr, l.kfp - l.ff);
+            if (rc) return rc;
+            act_done = true;
         }
         if (!act_done) {
             rc = product<OT>(m, opA, wp, l.w_gu, wp, m->G, 2 * l.ff, R, 2 * l.ff, wp, nullptr, 0);
@@ -1300,6 +1324,11 @@ int run_prenorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, const
             rc = seq_gemm_bf16_geglu(m->gp, opA, wp, l.w_gu, wp, opC, l.kfp, 0, R, 2 * l.ff, wp);
             if (rc > 0) return rc;
             if (rc == 0) { ctx().launches++; act_done = true; }
+        }
+        if (!act_done && R <= 8) {
+            rc = gated_rows<OT, 3>(opA, wp, l.w_gu, wp, opC, l.kfp, R, l.ff, wp, l.gu_inter, nullptr, 0);
+            if (rc) return rc;
+            act_done = true;
         }
         if (!act_done) {
             rc = product<OT>(m, opA, wp, l.w_gu, wp, m->G, 2 * l.ff, R, 2 * l.ff, wp, nullptr, 0);
@@ -1425,6 +1454,11 @@ int run_pass(gtb_seq_model* m, const PassTables& t, int R, int S, bool from_pend
                 rc = seq_gemm_bf16_geglu(m->gp, opB, wp, l.w_gu, wp, opC, l.kout_p, l.kout - l.ff, R, 2 * l.ff, wp);
                 if (rc > 0) return rc;
                 if (rc == 0) { ctx().launches++; ff_done = true; }
+            }
+            if (!ff_done && R <= 8) {
+                rc = gated_rows<OT, 3>(opB, wp, l.w_gu, wp, opC + (l.kout - l.ff), l.kout_p, R, l.ff, wp, l.gu_inter, nullptr, 0);
+                if (rc) return rc;
+                ff_done = true;
             }
             if (!ff_done) {
                 rc = product<OT>(m, opB, wp, l.w_gu, wp, m->G, 2 * l.ff, R, 2 * l.ff, wp, nullptr, 0);

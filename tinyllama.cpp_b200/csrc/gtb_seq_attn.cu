@@ -6,8 +6,8 @@
 // thread of warp 5 issues the products:
 //     S[128][64] = Q K^T      (Q staged once as bf16 in shared memory, K tile K-major)
 //     O[128][VP] += P V       (P bf16 from TMEM, V tile as it lies in the cache: rows of keys, the MN-major B operand)
-// There are two score buffers, and the weights of a tile replace its scores: while tile j's weights are computed, P V of tile j - 1 and the
-// scores of tile j + 1 run, so the weight threads hardly ever wait for a product's latency.
+// There are two score and two weight buffers: while tile j's weights are computed, the scores of tile j + 1 and P V of tile j - 1 run, so the
+// weight threads hardly ever wait for a product's latency.
 // The softmax keeps its reference maximum until a row's scores exceed it by 2^8 and only then rescales O in TMEM (a rare event, the only one
 // that waits for P V; weights up to 2^8 lose nothing in fp32 sums or bf16 operands).  Scores, weights, sums and the output are fp32, the
 // weights enter P V as bf16.
@@ -35,8 +35,11 @@ template <int DP, int VP> struct AtCfg {
     static constexpr int STAGES = DP + VP == 256 ? 2 : 3;      // (two CTAs per SM)
     static constexpr uint32_t Q_BYTES = 128 * DP * 2, K_BYTES = AT_KT * DP * 2, V_BYTES = AT_KT * VP * 2;
     static constexpr uint32_t SMEM = Q_BYTES + STAGES * (K_BYTES + V_BYTES) + 1024 + 256;
-    // TMEM columns: two score buffers (a tile's weights, two per column, replace its scores), output
-    static constexpr uint32_t COLS = 256, O_COL = 2 * AT_KT;
+    // TMEM columns: two score buffers, two weight buffers (two weights per column), output.  Values of 128 channels leave no room for weights of
+    // their own: there a tile's weights replace its scores
+    static constexpr bool P_OWN = VP == 64;
+    static constexpr uint32_t COLS = 256, O_COL = P_OWN ? 3 * AT_KT : 2 * AT_KT;
+    static __host__ __device__ constexpr uint32_t p_col(int j) { return P_OWN ? 2 * AT_KT + (j & 1) * (AT_KT / 2) : (j & 1) * AT_KT; }
     static_assert(O_COL + VP <= COLS, "TMEM columns");
     static constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(AT_KT >> 3) << 17) | (8u << 24);
     static constexpr uint32_t IDESC_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (8u << 17) | (8u << 24);      // B MN-major, N = 64
@@ -212,18 +215,19 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
             }
             if (!(ok = at_wait(p_bar(j), (j >> 1) & 1, abort_flag))) break;
             tc_fence_after();
+            if (Cfg::P_OWN && j + 2 < n_it && !(ok = scores(j + 2))) break;      // tile j's scores have been read: the next ones need not wait for P V
             if (lane == 0) {
                 const uint32_t sv = sm_v + s * Cfg::V_BYTES;
 #pragma unroll
                 for (int c = 0; c < VP / 64; c++)
 #pragma unroll
                     for (int k = 0; k < KT / 16; k++)
-                        umma_f16_ts(tm + Cfg::O_COL + c * 64, tm + (j & 1) * KT + k * 8, umma_desc_sw128(sv + c * (KT * 128) + k * 2048), Cfg::IDESC_O, j > 0 || k > 0);
+                        umma_f16_ts(tm + Cfg::O_COL + c * 64, tm + Cfg::p_col(j) + k * 8, umma_desc_sw128(sv + c * (KT * 128) + k * 2048), Cfg::IDESC_O, j > 0 || k > 0);
                 umma_commit(v_empty(s));
                 umma_commit(o_bar(j));
             }
             __syncwarp();
-            if (j + 2 < n_it) {     // the next scores replace the weights that this product reads
+            if (!Cfg::P_OWN && j + 2 < n_it) {     // the next scores replace the weights that this product reads
                 if (!(ok = at_wait(o_bar(j), (j >> 1) & 1, abort_flag))) break;
                 ok = scores(j + 2);
             }
@@ -320,6 +324,7 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
                     }
                 }
             }
+            if (Cfg::P_OWN && it > 1 && !(ok = at_wait(o_bar(it), ((it - 2) >> 1) & 1, abort_flag))) break;      // the product that read this weight buffer is done
             const float mu = m == -INFINITY ? 0.0f : m;
             float l0 = 0.0f, l1 = 0.0f;
 #pragma unroll
@@ -339,7 +344,7 @@ k_attn_tc(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUten
                     }
                     w[j] = at_pack(p0, p1);
                 }
-                tmem_st16(ts + c / 2, w);
+                tmem_st16(tl + Cfg::p_col(it) + c / 2, w);
             }
             l += l0 + l1;
             tmem_wait_st();

@@ -354,14 +354,25 @@ template <> __device__ __forceinline__ void load8<bf16>(const bf16* p, float (&v
 #pragma unroll
     for (int i = 0; i < 4; i++) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
 }
-// OUT float: C (fp32) as above.  GELU: gelu(A . W^T), erf form, as the next product's operand (OUT = AT) -- the activation of an ungated
-// feed-forward; no bias, no accumulation.
-template <typename AT, int MR, int NC, bool GELU = false, typename OUT = float>
+// where gate and up rows of activation c are placed: groups of 32 gate rows, each followed by its 32 up rows (inter), or all gates, then all ups
+__device__ __forceinline__ int gu_gate_row(int c, int inter) { return inter ? (c >> 5) * 64 + (c & 31) : c; }
+__device__ __forceinline__ int gu_up_row(int c, int ff, int inter) { return inter ? (c >> 5) * 64 + (c & 31) + 32 : ff + c; }
+// ACT 0: C (fp32) as above.  The others write the next product's operand (OUT = AT), without bias or accumulation: 1: gelu(A . W^T), erf form, the
+// activation of an ungated feed-forward; 2, 3: silu(gate) * up * row_w and gelu_tanh(gate) * up, N / 2 activations from N rows of gate and up (gu: how
+// they are placed, see gu_gate_row) -- a CTA owns NC / 2 of them.  (A kernel of its own for the activation costs 3.5 us a layer of a decode step.)
+template <typename AT, int MR, int NC, int ACT = 0, typename OUT = float>
 __global__ void __launch_bounds__(256) k_gemv_rows(const AT* __restrict__ A, int lda, const bf16* __restrict__ W, int ldw, OUT* __restrict__ C, int ldc,
-                                                   int M, int N, int K, const float* __restrict__ bias, int accumulate) {
+                                                   int M, int N, int K, const float* __restrict__ bias, int accumulate, int inter = 0) {
     __shared__ float red[8][MR * NC];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n0 = blockIdx.x * NC;
+    constexpr bool GATED = ACT >= 2;
+    const int n0 = blockIdx.x * (GATED ? NC / 2 : NC), n_out = GATED ? N / 2 : N;
+    // row of W behind accumulator column c (gated: the gates of the CTA's activations, then their ups), N when there is none
+    auto wrow = [&](int c) {
+        if (!GATED) return n0 + c < N ? n0 + c : N;
+        const int ch = n0 + c % (NC / 2);
+        return ch >= n_out ? N : c < NC / 2 ? gu_gate_row(ch, inter) : gu_up_row(ch, n_out, inter);
+    };
     float acc[MR][NC];
 #pragma unroll
     for (int m = 0; m < MR; m++)
@@ -374,7 +385,7 @@ __global__ void __launch_bounds__(256) k_gemv_rows(const AT* __restrict__ A, int
     auto fetch = [&](int kk) {
 #pragma unroll
         for (int c = 0; c < NC; c++)
-            wn[c] = (n0 + c < N) ? __ldg(reinterpret_cast<const uint4*>(W + (size_t)(n0 + c) * ldw + kk)) : make_uint4(0, 0, 0, 0);
+            wn[c] = wrow(c) < N ? __ldg(reinterpret_cast<const uint4*>(W + (size_t)wrow(c) * ldw + kk)) : make_uint4(0, 0, 0, 0);
     };
     if (k < K) fetch(k);
     pdl_trigger_and_wait();
@@ -407,13 +418,27 @@ __global__ void __launch_bounds__(256) k_gemv_rows(const AT* __restrict__ A, int
             if (lane == 0) red[warp][m * NC + c] = v;
         }
     __syncthreads();
-    if (threadIdx.x < MR * NC) {
+    if constexpr (GATED) {
+        if (threadIdx.x < MR * NC / 2) {
+            const int m = threadIdx.x / (NC / 2), c = threadIdx.x % (NC / 2);
+            if (m < M && n0 + c < n_out) {
+                float gt = 0.0f, up = 0.0f;
+#pragma unroll
+                for (int w = 0; w < 8; w++) { gt += red[w][m * NC + c]; up += red[w][m * NC + NC / 2 + c]; }
+                const float v = ACT == 2 ? (bias ? bias[m] : 1.0f) * (gt * sigmoidf_(gt)) * up : gelu_tanh(gt) * up;      // (bias: the rows' weights)
+                C[(size_t)m * ldc + n0 + c] = cvt<OUT>(v);
+            }
+        }
+        // the operand's padding, which meets zero weights
+        if (blockIdx.x == 0 && accumulate > 0 && threadIdx.x < accumulate)
+            for (int m = 0; m < M; m++) C[(size_t)m * ldc + n_out + threadIdx.x] = cvt<OUT>(0.0f);
+    } else if (threadIdx.x < MR * NC) {
         const int m = threadIdx.x / NC, c = threadIdx.x % NC;
         if (m < M && n0 + c < N) {
             float o = 0.0f;
 #pragma unroll
             for (int w = 0; w < 8; w++) o += red[w][threadIdx.x];
-            if constexpr (GELU) {
+            if constexpr (ACT == 1) {
                 C[(size_t)m * ldc + n0 + c] = cvt<OUT>(gelu_erf(o));
             } else {
                 if (bias) o += bias[n0 + c];

@@ -226,9 +226,11 @@ __global__ void __launch_bounds__(128) k_lat_qrot(PassTables t, LatAttn b, const
     const float* q = Q + (size_t)r * ldq + q0;
     float* o = QR + (size_t)r * ld_qr;
     const int half = b.rot_dims / 2;
-    for (int e = threadIdx.x; e < b.heads * hd; e += blockDim.x) {
-        const int h = e / hd, i = e % hd, j = i - b.dim;
-        if (j < 0 || j >= b.rot_dims) { if (o + e != q + e) o[e] = q[e]; continue; }
+    // in place only the rotated pairs are touched
+    const int first_e = o == q ? b.dim : 0, per = o == q ? b.rot_dims : hd;
+    for (int e0 = threadIdx.x; e0 < b.heads * per; e0 += blockDim.x) {
+        const int h = e0 / per, i = first_e + e0 - h * per, j = i - b.dim, e = h * hd + i;
+        if (j < 0 || j >= b.rot_dims) { o[e] = q[e]; continue; }
         const int pr = b.rot_layout ? j >> 1 : (j < half ? j : j - half);
         const bool first = b.rot_layout ? (j & 1) == 0 : j < half;
         if (!first) continue;                     // the pair's first entry writes both
@@ -241,6 +243,11 @@ __global__ void __launch_bounds__(128) k_lat_qrot(PassTables t, LatAttn b, const
         o[h * hd + b.dim + i0] = u * cs - v * sn;
         o[h * hd + b.dim + i1] = v * cs + u * sn;
     }
+}
+
+__device__ __forceinline__ uint2 lat_pack4(const float4& v) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
 // Expanded keys and values of n cached tokens of one slot from position lo: X [n][heads * (dim + vdim)] (fp32) holds [uk c | uv c];
@@ -544,11 +551,6 @@ __global__ void __launch_bounds__(32) k_moe_route_sigmoid(const float* __restric
     for (int k = lane; k < top; k += 32) sel_w[(size_t)r * top + k] *= inv;
     if (shared_w && lane == 0) shared_w[r] = sigmoidf_(z[n_exp]);
 }
-
-// rows of the fused [gate | up] matrix of a gated feed-forward: plain = ff gate rows then ff up rows; interleaved = groups of 32 gate
-// rows each followed by their 32 up rows (what the tensor-core epilogue reads)
-__device__ __forceinline__ int gu_gate_row(int c, int inter) { return inter ? (c >> 5) * 64 + (c & 31) : c; }
-__device__ __forceinline__ int gu_up_row(int c, int ff, int inter) { return inter ? (c >> 5) * 64 + (c & 31) + 32 : ff + c; }
 
 // Few rows: pair (row r, choice k) with expert e streams that expert's gate and up rows once: act[pair][c] = w * silu(gate_e[c] . x_r) *
 // (up_e[c] . x_r) for c < ff, zero up to the padded width kfp.  grid (R * top, column groups); a warp takes one column at a time.
