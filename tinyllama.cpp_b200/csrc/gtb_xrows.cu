@@ -221,16 +221,18 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f
 // The epilogue of one (row, 64-column tile n) for one warp: lane = column inside each 32-block (v[0]: column 64 n + lane, v[1]: column
 // 64 n + 32 + lane; gate|up: gate channel 32 n + lane and up channel 32 n + lane), every re-encode is warp-local.  Shared by the SIMT
 // GEMM (accumulators in registers) and the tensor-core GEMM's epilogue kernel (accumulated rows read back from HBM).
+// 32-column block n of a row: x = E(x + E(linear output)), lane = column
+__device__ __forceinline__ void xr_res_store(const XrGemmArgs& a, int row, int n, int lane, float v) {
+    float* px = a.res + (size_t)row * a.E + 32 * n + lane;
+    const float d1 = q8_roundtrip_lane(v);
+    *px = q8_roundtrip_lane(__fadd_rn(*px, d1));
+}
 template <int EPI>
 __device__ __forceinline__ void xr_epilogue(const XrGemmArgs& a, int row, const XrRow& rw, int n, int lane, const float (&v)[2], bool store_logits) {
     if (EPI == XEPI_RES) {
         // Residual (gten/ops.h:870-898): x = E(x + E(linear output))
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-            float* px = a.res + (size_t)row * a.E + 64 * n + 32 * c + lane;
-            const float d1 = q8_roundtrip_lane(v[c]);
-            *px = q8_roundtrip_lane(__fadd_rn(*px, d1));
-        }
+        xr_res_store(a, row, 2 * n, lane, v[0]);
+        xr_res_store(a, row, 2 * n + 1, lane, v[1]);
     } else if (EPI == XEPI_SILU) {
         // gten/modules.cpp:238-247: E(E(silu(E(gate))) * E(up))
         const float g1 = q8_roundtrip_lane(v[0]);
@@ -288,36 +290,39 @@ __device__ __forceinline__ void xr_epilogue(const XrGemmArgs& a, int row, const 
     }
 }
 
-// NW warps per CTA, TR = 16 / NW rows per warp: (4, 4) amortises a weight block over 4 rows (fewest instructions; large N),
-// (8, 2) doubles the warps per tile for the matrices with few column tiles (N <= 2560: q|k|v, o, down)
-template <int WT, int EPI, int NW, int NS = XG_STAGES, int MINB = (NW == 4) ? 4 : 2>
+// NW warps per CTA, TR rows per warp, NC columns per lane (2; 1 only where a lane needs no partner 32 columns on: the residual epilogue).  More rows and
+// columns per warp amortise a weight block's unpacking (fewest instructions per output: large passes), fewer spread a small pass over more
+// warps and CTAs: a (row, column) chain is 64 or 176 dependent blocks long whatever the shape, so a pass of a few rows is bound by how many
+// instructions its busiest scheduler issues.  launch_gemm picks the shape.
+template <int WT, int EPI, int NW, int TR, int NC = 2, int NS = XG_STAGES, int MINB = (NW == 4) ? 4 : (NW * TR == 8) ? 3 : 2>
 __global__ void __launch_bounds__(NW * 32, MINB) k_xr_gemm(XrGemmArgs a) {
-    constexpr int XG_NT = NW * 32, TR = XG_BM / NW;
+    constexpr int XG_NT = NW * 32, BM = NW * TR, BN = 32 * NC;
+    static_assert(BM <= XG_BM && (NC == 2 || EPI == XEPI_RES), "tile");
     extern __shared__ __align__(16) unsigned char smem[];
     XgStage<WT>* stages = reinterpret_cast<XgStage<WT>*>(smem);
     constexpr int WB = XgStage<WT>::WB, WPC = XG_KC * WB;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int n = blockIdx.x;
-    const int rbase = a.row0 + blockIdx.y * XG_BM, rend = a.row0 + a.n_rows;
+    const int rbase = a.row0 + blockIdx.y * BM, rend = a.row0 + a.n_rows;
     const int nb = a.nb, nchunk = nb / XG_KC;
     // weight row of local column c: plain tiles are 64 consecutive rows; gate|up tiles are 32 gate rows + the same 32 up rows
     auto wrow = [&](int c) -> int {
-        int r = (EPI == XEPI_SILU) ? ((c < 32) ? 32 * n + c : a.up_off + 32 * n + c - 32) : 64 * n + c;
+        int r = (EPI == XEPI_SILU) ? ((c < 32) ? 32 * n + c : a.up_off + 32 * n + c - 32) : BN * n + c;
         return min(r, a.N - 1);
     };
     auto load_weights = [&](int s, int kc) {
         XgStage<WT>& st = stages[s];
 #pragma unroll
-        for (int i = tid; i < XG_BN * WPC; i += XG_NT) {
+        for (int i = tid; i < BN * WPC; i += XG_NT) {
             const int c = i / WPC, j = i % WPC;
             cp_async16(&st.wd[c][j], a.wd + ((size_t)wrow(c) * nb + (size_t)kc * XG_KC) * WB + j, true);
         }
-        if (tid < XG_BN) cp_async16(&st.ws[tid], a.ws + (size_t)wrow(tid) * nb + (size_t)kc * XG_KC, true);
+        if (tid < BN) cp_async16(&st.ws[tid], a.ws + (size_t)wrow(tid) * nb + (size_t)kc * XG_KC, true);
     };
     auto load_act = [&](int s, int kc) {
         XgStage<WT>& st = stages[s];
 #pragma unroll
-        for (int i = tid; i < XG_BM * XG_KC * 4; i += XG_NT) {
+        for (int i = tid; i < BM * XG_KC * 4; i += XG_NT) {
             const int r = i >> 5, j = i & 31;
             const int gr = rbase + r;
             const bool ok = gr < rend;
@@ -325,11 +330,11 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_xr_gemm(XrGemmArgs a) {
             cp_async16(reinterpret_cast<uint4*>(&st.act[r][0]) + j, src, ok);
         }
     };
-    f32x2 acc[TR][2][2];                                             // lanes (0, 1) and (2, 3) of each (row, column)
+    f32x2 acc[TR][NC][2];                                             // lanes (0, 1) and (2, 3) of each (row, column)
 #pragma unroll
     for (int r = 0; r < TR; r++)
 #pragma unroll
-        for (int c = 0; c < 2; c++) { acc[r][c][0] = pk2(0.0f, 0.0f); acc[r][c][1] = pk2(0.0f, 0.0f); }
+        for (int c = 0; c < NC; c++) { acc[r][c][0] = pk2(0.0f, 0.0f); acc[r][c][1] = pk2(0.0f, 0.0f); }
     // weights never depend on the previous kernel of the chain: their first chunks are in flight before it has finished
 #pragma unroll
     for (int s = 0; s < NS - 1; s++)
@@ -340,6 +345,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_xr_gemm(XrGemmArgs a) {
         if (s < nchunk) load_act(s, s);
         cp_async_commit();
     }
+    const bool active = rbase + wid * TR < rend;                     // (warps without a row only help to load)
     for (int kc = 0; kc < nchunk; kc++) {
         cp_async_wait<NS - 2>();
         __syncthreads();
@@ -348,29 +354,30 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_xr_gemm(XrGemmArgs a) {
             load_act((kc + NS - 1) % NS, kc + NS - 1);
         }
         cp_async_commit();
+        if (!active) continue;
         const XgStage<WT>& st = stages[kc % NS];
-        const uint4 sA = st.ws[lane], sB = st.ws[lane + 32];
+        const uint4 sA = st.ws[lane], sB = st.ws[NC == 2 ? lane + 32 : lane];
         const __half* hA = reinterpret_cast<const __half*>(&sA);
         const __half* hB = reinterpret_cast<const __half*>(&sB);
 #pragma unroll
         for (int b = 0; b < XG_KC; b++) {
             // the two columns' blocks: wx = codes paired with the activation's X words, wy with its Y words
-            uint32_t wx[2][4], wy[2][4];
+            uint32_t wx[NC][4], wy[NC][4];
             if (WT == DT_Q4) {
-                const uint4 w0 = st.wd[lane][b], w1 = st.wd[lane + 32][b];
-                const uint32_t r0[4] = {w0.x, w0.y, w0.z, w0.w}, r1[4] = {w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-                for (int l = 0; l < 4; l++) {
-                    wx[0][l] = (r0[l] >> 4) & 0x0f0f0f0fu; wy[0][l] = r0[l] & 0x0f0f0f0fu;
-                    wx[1][l] = (r1[l] >> 4) & 0x0f0f0f0fu; wy[1][l] = r1[l] & 0x0f0f0f0fu;
+                for (int c = 0; c < NC; c++) {
+                    const uint4 w = st.wd[lane + 32 * c][b];
+                    const uint32_t rr[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                    for (int l = 0; l < 4; l++) { wx[c][l] = (rr[l] >> 4) & 0x0f0f0f0fu; wy[c][l] = rr[l] & 0x0f0f0f0fu; }
                 }
             } else {
-                const uint4 x0 = st.wd[lane][2 * b], y0 = st.wd[lane][2 * b + 1];
-                const uint4 x1 = st.wd[lane + 32][2 * b], y1 = st.wd[lane + 32][2 * b + 1];
-                wx[0][0] = x0.x; wx[0][1] = x0.y; wx[0][2] = x0.z; wx[0][3] = x0.w;
-                wy[0][0] = y0.x; wy[0][1] = y0.y; wy[0][2] = y0.z; wy[0][3] = y0.w;
-                wx[1][0] = x1.x; wx[1][1] = x1.y; wx[1][2] = x1.z; wx[1][3] = x1.w;
-                wy[1][0] = y1.x; wy[1][1] = y1.y; wy[1][2] = y1.z; wy[1][3] = y1.w;
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    const uint4 x = st.wd[lane + 32 * c][2 * b], y = st.wd[lane + 32 * c][2 * b + 1];
+                    wx[c][0] = x.x; wx[c][1] = x.y; wx[c][2] = x.z; wx[c][3] = x.w;
+                    wy[c][0] = y.x; wy[c][1] = y.y; wy[c][2] = y.z; wy[c][3] = y.w;
+                }
             }
             const float dw[2] = {__half2float(hA[b]), __half2float(hB[b])};
 #pragma unroll
@@ -386,7 +393,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_xr_gemm(XrGemmArgs a) {
                 }
                 const float ad = ab.d;
 #pragma unroll
-                for (int c = 0; c < 2; c++) {
+                for (int c = 0; c < NC; c++) {
                     // s = da * dw has <= 22 significant bits, so XB_M * s is exact and fmaf((M + l), s, -M s) is the
                     // single rounding of l * s: exactly `(float)lane * (da * dw)` of ops.h:282-287
                     const float s = __fmul_rn(ad, dw[c]);
@@ -412,12 +419,13 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_xr_gemm(XrGemmArgs a) {
         if (rw.slot < 0) continue;
         float v[2];
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
+        for (int c = 0; c < NC; c++) {
             float a0, a1, a2, a3;
             unpk2(acc[r][c][0], a0, a1); unpk2(acc[r][c][1], a2, a3);
             v[c] = __fadd_rn(__fadd_rn(a0, a1), __fadd_rn(a2, a3));
         }
-        xr_epilogue<EPI>(a, row, rw, n, lane, v, true);
+        if constexpr (NC == 1) xr_res_store(a, row, n, lane, v[0]);
+        else xr_epilogue<EPI>(a, row, rw, n, lane, v, true);
     }
 }
 
@@ -1223,26 +1231,41 @@ cudaError_t xr_launch(void (*kern)(KArgs...), dim3 grid, int block, size_t smem,
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-template <int WT, int EPI, int NW, int NS = XG_STAGES, int MINB = (NW == 4) ? 4 : 2>
+template <int WT, int EPI, int NW, int TR, int NC = 2, int NS = XG_STAGES, int MINB = (NW == 4) ? 4 : (NW * TR == 8) ? 3 : 2>
 int launch_gemm_nw(const XrGemmArgs& a, int n_tiles) {
     const size_t smem = sizeof(XgStage<WT>) * NS;
     static bool attr = false;
     if (!attr) {
-        GTB_CUDA(cudaFuncSetAttribute(k_xr_gemm<WT, EPI, NW, NS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        GTB_CUDA(cudaFuncSetAttribute(k_xr_gemm<WT, EPI, NW, TR, NC, NS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr = true;
     }
-    dim3 grid(n_tiles, (a.n_rows + XG_BM - 1) / XG_BM);
-    GTB_CUDA(xr_launch(k_xr_gemm<WT, EPI, NW, NS, MINB>, grid, NW * 32, smem, a));
+    dim3 grid(n_tiles * (NC == 1 ? 2 : 1), (a.n_rows + NW * TR - 1) / (NW * TR));
+    GTB_CUDA(xr_launch(k_xr_gemm<WT, EPI, NW, TR, NC, NS, MINB>, grid, NW * 32, smem, a));
     GTB_LAUNCHED();
     return GTB_OK;
 }
+// Shapes by the pass's rows (6-layer passes, us, Q4 / Q8): residual Linears (32 column tiles only) on single rows and columns, 8 rows 587 -> 534 / 603 -> 529,
+// 16 rows 754 -> 593 / 713 -> 564, on two rows and single columns 24 rows 887 -> 793 / 908 -> 818, 33 rows 918 -> 875 / 957 -> 918, level at 48; gate | up on one or
+// two rows per warp instead of four, 4 rows 604 -> 485 / 618 -> 500, 16 rows 754 -> 718 / 713 -> 702, 33 rows 918 -> 875 / 957 -> 930, level at 48;
+// q | k | v on one row per warp, 8 rows 587 -> 564 / 603 -> 589, 16 rows 754 -> 693 / 713 -> 690, level at 33.
 template <int WT, int EPI>
 int launch_gemm(const XrGemmArgs& a, int n_tiles) {
+    const int R = a.n_rows;
+    if constexpr (EPI == XEPI_RES) {
+        if (R <= 16) return launch_gemm_nw<WT, EPI, 4, 1, 1>(a, n_tiles);
+        if (R <= 40) return launch_gemm_nw<WT, EPI, 8, 2, 1>(a, n_tiles);
+    } else if constexpr (EPI == XEPI_QKV) {
+        if (R <= 12) return launch_gemm_nw<WT, EPI, 4, 1>(a, n_tiles);
+        if (R <= 24) return launch_gemm_nw<WT, EPI, 8, 1>(a, n_tiles);
+    } else {
+        if (R <= 4) return launch_gemm_nw<WT, EPI, 4, 1>(a, n_tiles);
+        if (R <= 40) return launch_gemm_nw<WT, EPI, 4, 2>(a, n_tiles);
+    }
     // few column tiles: 8 warps x 2 rows per tile keep two warps per scheduler busy; many tiles: 4 warps x 4 rows
-    const int ctas = n_tiles * ((a.n_rows + XG_BM - 1) / XG_BM);
-    if (EPI != XEPI_SILU && EPI != XEPI_HEAD && ctas <= 2 * ctx().sm_count) return launch_gemm_nw<WT, EPI, 8>(a, n_tiles);
-    if (g_xr_variant == 1 && (EPI == XEPI_SILU || EPI == XEPI_HEAD)) return launch_gemm_nw<WT, EPI, 4, 2, 5>(a, n_tiles);   // 2 stages, 5 CTAs / SM
-    return launch_gemm_nw<WT, EPI, 4>(a, n_tiles);
+    const int ctas = n_tiles * ((R + XG_BM - 1) / XG_BM);
+    if (EPI != XEPI_SILU && EPI != XEPI_HEAD && ctas <= 2 * ctx().sm_count) return launch_gemm_nw<WT, EPI, 8, 2>(a, n_tiles);
+    if (g_xr_variant == 1 && (EPI == XEPI_SILU || EPI == XEPI_HEAD)) return launch_gemm_nw<WT, EPI, 4, 4, 2, 2, 5>(a, n_tiles);   // 2 stages, 5 CTAs / SM
+    return launch_gemm_nw<WT, EPI, 4, 4>(a, n_tiles);
 }
 
 // ---- tensor-core Linear (gtb_xtensor.cuh): rows per thread chosen so that the (tile, row group) units fill the SMs
