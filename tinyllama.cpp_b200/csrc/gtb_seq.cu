@@ -50,6 +50,10 @@ using namespace gtb::seq;
 namespace {
 
 inline int pad64(int k) { return (k + 63) / 64 * 64; }
+// CTAs per row of k_sattn_prep, whose warps walk a row's heads: a CTA for every four heads on passes of few rows, where latency counts; one per row
+// once the rows alone fill the chip, so that a row's rotation is computed once per warp and not per head (gated attention, 2 x 2048 rows: 655 -> 636 us
+// a pass together with the embedding's registers; the head-wise kernels without a rotation lose by it)
+inline int unit_ctas(int R, int full) { return std::max(1, std::min(full, 2048 / std::max(1, R))); }
 constexpr int SPLIT_MAX_ROWS = 64;          // passes of at most this many rows may split a row's keys over several CTAs
 
 struct TensorDest {
@@ -503,7 +507,7 @@ int run_postnorm_layer(gtb_seq_model* m, const PassTables& t, int R, int S, cons
         }
     } else {
         const SoftAttn a = soft_args(m, b, run);
-        pdl_launch(k_sattn_prep<OT>, dim3(R, (a.heads + 2 * a.kv_heads + 3) / 4), 128, 0, st, t, a, m->P, l.n1, (OT*)run.kc[0], (OT*)run.vc[0]);
+        pdl_launch(k_sattn_prep<OT>, dim3(R, unit_ctas(R, (a.heads + 2 * a.kv_heads + 3) / 4)), 128, 0, st, t, a, m->P, l.n1, (OT*)run.kc[0], (OT*)run.vc[0]);
         GTB_LAUNCHED();
         if (a.pool > 0) {
             pdl_launch(k_pool_update<OT>, R, 128, 0, st, t, a, (const OT*)run.kc[0], (const OT*)run.vc[0], run.pk, run.pv);
@@ -736,7 +740,7 @@ int run_soft_branch(gtb_seq_model* m, const PassTables& t, int R, int S, const R
         Q = m->convQ; ldq = b.kq;
         a.q_off = 0; a.gate_src = m->P; a.gate_ld = l.n1;
     } else {
-        pdl_launch(k_sattn_prep<OT>, dim3(R, (units + nk + nv + 3) / 4), 128, 0, st, t, a, m->P, l.n1, (OT*)run.kc[bi], (OT*)run.vc[bi]);
+        pdl_launch(k_sattn_prep<OT>, dim3(R, unit_ctas(R, (units + nk + nv + 3) / 4)), 128, 0, st, t, a, m->P, l.n1, (OT*)run.kc[bi], (OT*)run.vc[bi]);
         GTB_LAUNCHED();
     }
     // two maps per head: the units' outputs stay fp32 (their difference is taken afterwards), unit-major in m->O

@@ -371,6 +371,11 @@ __global__ void __launch_bounds__(128) k_sattn_prep(PassTables t, SoftAttn b, fl
     const size_t crow = (size_t)slot * b.max_ctx + pos;
     const int M = sa_maps(b), nq = b.heads * M, nk = b.own_kv ? b.kv_heads * M : 0, nkv = b.own_kv && !b.v_is_k ? b.kv_heads : 0, half = b.rot_dims / 2;
     const float fpos = (float)pos;
+    // the row's rotation, the same for every head: a lane's first two pairs stay in registers over its units
+    float rcs[2], rsn[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+        if (lane + 32 * j < half) { sincosf(fpos * b.inv_freq[lane + 32 * j], &rsn[j], &rcs[j]); rsn[j] *= b.rot_amp; rcs[j] *= b.rot_amp; }
     for (int u = blockIdx.y * nw + wid; u < nq + nk + nkv; u += gridDim.y * nw) {
         if (u < nq + nk) {
             const bool is_q = u < nq;
@@ -390,8 +395,8 @@ __global__ void __launch_bounds__(128) k_sattn_prep(PassTables t, SoftAttn b, fl
                 const int i0 = b.rot_layout ? 2 * pr : pr, i1 = b.rot_layout ? 2 * pr + 1 : pr + half;
                 const float a = v[i0] * sc * (wn ? wn[i0] : 1.0f), c = v[i1] * sc * (wn ? wn[i1] : 1.0f);
                 float sn, cs;
-                sincosf(fpos * b.inv_freq[pr], &sn, &cs);
-                sn *= b.rot_amp; cs *= b.rot_amp;
+                if (pr < 64) { const int j = pr >> 5; sn = j ? rsn[1] : rsn[0]; cs = j ? rcs[1] : rcs[0]; }
+                else { sincosf(fpos * b.inv_freq[pr], &sn, &cs); sn *= b.rot_amp; cs *= b.rot_amp; }
                 const float ra = a * cs - c * sn, rc = c * cs + a * sn;
                 if (is_q) { v[i0] = ra; v[i1] = rc; } else { dst[i0] = cvt<OT>(ra); dst[i1] = cvt<OT>(rc); }
             }
