@@ -1145,7 +1145,8 @@ __global__ void __launch_bounds__(XA_NT) k_xf_attn_head(XfAttnArgs a) {
 // ---------------------------------------------------------------- host side
 // Programmatic dependent launch between the kernels of a pass.  Measured (tools/xrows_probe.py --pdl 0/1, same box): it helps the
 // latency-bound small passes (8 rows: 2.66 vs 2.76 ms per step) and costs 17 % on full ones (64 rows: 4.58 vs 3.91 ms: the early
-// resident CTAs of the next kernel take SM resources from the tail of the running one), so it is used for passes of <= 16 rows.
+// resident CTAs of the next kernel take SM resources from the tail of the running one), so it is used for passes of <= 16 rows, and
+// up to 40 rows where the Linears run on the small tiles (Q4 / Q8; eight prompts of 8 to 40 rows and 12 steps of 8: 35.6 -> 33.7 ms).
 static bool g_xr_pdl = true;
 static bool g_xr_pdl_now = false;
 static int g_xr_variant = 0;        // experiment switch for the large-N GEMM configuration
@@ -1319,7 +1320,7 @@ int run_pass(XrPlan* p, const XrModel& m, const XrKV& kv, const XrSeq& sq, const
              int head_rows, int eos_id, float* d_logits) {
     const gtb_model_config& c = m.cfg;
     const int E = c.n_embd, F = c.n_ffn, KVD = 64 * c.n_groups, R = plan.n_rows;
-    g_xr_pdl_now = g_xr_pdl && R <= 16 && !g_xr_tensor;      // the tensor-core kernels do not carry the dependent-launch protocol
+    g_xr_pdl_now = g_xr_pdl && R <= 40 && !g_xr_tensor;      // the tensor-core kernels do not carry the dependent-launch protocol
     GTB_CUDA(xr_launch(k_xr_plan, dim3(1), XR_MAX_ROWS, 0, plan));
     GTB_LAUNCHED();
     const size_t norm_smem = (size_t)E * 8;
