@@ -6,8 +6,8 @@ namespace gtb {
 namespace seq {
 
 struct SeqGemmPlan;
-// One attention branch over the rows of a pass: unit u (query part of a head) of row r attends keys of cache column block (u / (units per K/V
-// head ..)) under its own mask; see PassTables / SoftAttn for the meaning of the tables and of the shared fields.
+// One attention branch over the rows of a pass: unit u = head * maps + map of a row attends the keys of its K/V head (and map) and that head's
+// values under the row's own mask; see PassTables / SoftAttn for the meaning of the tables and of the shared fields.
 struct AttnTc {
     const int *seg_slot, *seg_row0, *seg_len, *row_pos;      // tables of the pass, S segments
     int S;
